@@ -304,16 +304,33 @@ __device__ void line_thomas(const Level<T>& L, T* x, const T* b, T* work,
   }
 }
 
+// x (and the first Chebyshev direction) of cell c, whose rhs is `b`, by `zero`.
+// START is whether its kind is a smoothing step, fixed at compile time: as a
+// run-time choice it slowed the line levels' restriction and entry (MG
+// application at 256^3 2.917 -> 2.956 ms, with it 2.929).
+template <bool START, class T>
+__device__ __forceinline__ void write_zero_start(const ZeroStart<T>& zero, T b, T* x, int c,
+                                                 int parity) {
+  if (!START) {
+    if (zero.kind != kZeroNone) x[c] = T(0);
+    return;
+  }
+  T d;
+  x[c] = zero_start_value<T>(zero.kind, zero.factor, b, zero.diag[c], parity, d);
+  if (zero.direction != nullptr) zero.direction[c] = d;
+}
+
 // Fused retained defect + restriction (apply_level_defect followed by
 // restrict_residual, src/solver_mg.cpp:3633-3721): every coarse cell sums
-// the defects of its children in dz, dy, dx order; coarse x is zeroed.
+// the defects of its children in dz, dy, dx order; coarse x starts by `zero`.
 // Fused defect + restriction: one block per coarse x-row (blockIdx.x;
 // blockIdx.y splits long rows), one coarse cell per thread, the coarsening
-// mask fixed at compile time; coarse x is zeroed.  Fine x and b in layout hx.
-template <class T, int MASK>
+// mask fixed at compile time.  Fine x and b in layout hx.
+template <class T, int MASK, bool START>
 __global__ void __launch_bounds__(kRowThreads)
     k_defect_restrict(Level<T> F, const T* __restrict__ x, const T* __restrict__ b, Level<T> C,
-                      T* __restrict__ cb, T* __restrict__ cx, int hx, int hxc) {
+                      T* __restrict__ cb, T* __restrict__ cx, int hx, int hxc,
+                      ZeroStart<T> zero) {
   grid_dependency_sync();
   const int row = blockIdx.x;
   const int ci = blockIdx.y * blockDim.x + threadIdx.x;
@@ -321,12 +338,13 @@ __global__ void __launch_bounds__(kRowThreads)
   const int ck = row / C.ny;
   const int cj = row - ck * C.ny;
   const int cc = hxc == 0 ? ci + C.nx * row : SplitPos{C.ny, hxc}(0, ci, cj, ck);
-  cb[cc] = hx == 0
-               ? defect_restrict_at<T, PlainLoad, NaturalPos, MASK>(F, x, b, MASK, ci, cj, ck,
-                                                                   NaturalPos())
-               : defect_restrict_at<T, PlainLoad, SplitPos, MASK>(F, x, b, MASK, ci, cj, ck,
-                                                                 SplitPos{F.ny, hx});
-  cx[cc] = T(0);
+  const T sum = hx == 0
+                    ? defect_restrict_at<T, PlainLoad, NaturalPos, MASK>(F, x, b, MASK, ci, cj,
+                                                                        ck, NaturalPos())
+                    : defect_restrict_at<T, PlainLoad, SplitPos, MASK>(F, x, b, MASK, ci, cj, ck,
+                                                                      SplitPos{F.ny, hx});
+  cb[cc] = sum;
+  write_zero_start<START>(zero, sum, cx, cc, (ci + cj + ck) & 1);
 }
 
 // Trilinear prolongation and add, zero on solid cells (prolongate_cell).
@@ -484,18 +502,20 @@ __global__ void k_coarse_solve(Level<TC> L, T* x, const T* b, TC* xs, TC* bs,
 
 // ---------------------------------------------------------------------------
 // MG entry/exit (apply_impl, src/solver_mg.cpp:4866-4878, 5078-5117).
-template <class T>
+template <class T, bool START>
 __global__ void k_mg_enter(int n, const double* __restrict__ r,
                            const uint8_t* __restrict__ active,
-                           T* __restrict__ b, T* __restrict__ x, VecLayout v, bool zero_x) {
+                           T* __restrict__ b, T* __restrict__ x, VecLayout v,
+                           ZeroStart<T> zero) {
   grid_dependency_sync();
   // A warp per x-row: the split position of a cell is then the row's base
   // plus its parity half, with no division per cell.
   for_each_cell_by_rows(v.nx, v.ny, n / (v.nx * v.ny), [&](int i, int j, int k, int c) {
     const bool on = active == nullptr || active[c] != 0;
     const int at = v.hx == 0 ? c : 2 * v.hx * (j + v.ny * k) + (i & 1) * v.hx + (i >> 1);
-    b[at] = on ? static_cast<T>(r[c]) : T(0);
-    if (zero_x) x[at] = T(0);
+    const T value = on ? static_cast<T>(r[c]) : T(0);
+    b[at] = value;
+    write_zero_start<START>(zero, value, x, at, (i + j + k) & 1);
   });
 }
 
@@ -1560,13 +1580,19 @@ void launch_chebyshev_stage(cudaStream_t s, const Level<T>& L, const T* x,
 template <class T>
 void launch_defect_restrict(cudaStream_t s, const Level<T>& F, const T* x,
                             const T* b, const Level<T>& C, T* cb, T* cx,
-                            int mask, int hx, int hxc) {
+                            int mask, int hx, int hxc, const ZeroStart<T>& zero) {
   int threads = 0;
   const dim3 grid = row_grid(C.ny * C.nz, C.nx, threads);
+  const bool start = zero.kind == kZeroChebyshev || zero.kind == kZeroRedBlack;
   switch (mask & 7) {
 #define HFPS_RESTRICT_CASE(M)                                                              \
   case M:                                                                                  \
-    launch(k_defect_restrict<T, M>, grid, threads, 0, s, F, x, b, C, cb, cx, hx, hxc);     \
+    if (start)                                                                             \
+      launch(k_defect_restrict<T, M, true>, grid, threads, 0, s, F, x, b, C, cb, cx, hx, hxc, \
+             zero);                                                                        \
+    else                                                                                   \
+      launch(k_defect_restrict<T, M, false>, grid, threads, 0, s, F, x, b, C, cb, cx, hx, hxc, \
+             zero);                                                                        \
     break;
     HFPS_RESTRICT_CASE(0) HFPS_RESTRICT_CASE(1) HFPS_RESTRICT_CASE(2) HFPS_RESTRICT_CASE(3)
     HFPS_RESTRICT_CASE(4) HFPS_RESTRICT_CASE(5) HFPS_RESTRICT_CASE(6) HFPS_RESTRICT_CASE(7)
@@ -1606,8 +1632,11 @@ void launch_coarse_solve(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
 }
 template <class T>
 void launch_mg_enter(cudaStream_t s, int n, const double* r,
-                     const uint8_t* active, T* b, T* x, VecLayout v, bool zero_x) {
-  launch(k_mg_enter<T>, grid_for(n), kThreads, 0, s, n, r, active, b, x, v, zero_x);
+                     const uint8_t* active, T* b, T* x, VecLayout v, const ZeroStart<T>& zero) {
+  if (zero.kind == kZeroChebyshev || zero.kind == kZeroRedBlack)
+    launch(k_mg_enter<T, true>, grid_for(n), kThreads, 0, s, n, r, active, b, x, v, zero);
+  else
+    launch(k_mg_enter<T, false>, grid_for(n), kThreads, 0, s, n, r, active, b, x, v, zero);
 }
 template <class T>
 void launch_mg_exit(cudaStream_t s, int n, const T* x, const uint8_t* active,
@@ -1896,11 +1925,12 @@ void launch_adjoint_source(cudaStream_t s, int n, const double* dl_dp,
                                           const T*, T*, T*, T, T, int);            \
   template void launch_defect_restrict<T>(cudaStream_t, const Level<T>&, const T*, \
                                           const T*, const Level<T>&, T*, T*, int,  \
-                                          int, int);                               \
+                                          int, int, const ZeroStart<T>&);          \
   template void launch_prolongate<T>(cudaStream_t, const Level<T>&, T*,            \
                                      const Level<T>&, const T*, int, int, int);    \
   template void launch_mg_enter<T>(cudaStream_t, int, const double*,               \
-                                   const uint8_t*, T*, T*, VecLayout, bool);       \
+                                   const uint8_t*, T*, T*, VecLayout,              \
+                                   const ZeroStart<T>&);                           \
   template void launch_mg_exit<T>(cudaStream_t, int, const T*, const uint8_t*,     \
                                   const double*, double*, VecLayout);              \
   template void launch_mg_exit_dot<T>(cudaStream_t, int, const T*, const uint8_t*, \

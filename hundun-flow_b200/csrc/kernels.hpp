@@ -85,11 +85,24 @@ template <class T>
 void launch_chebyshev_stage(cudaStream_t s, const Level<T>& L, const T* x,
                             const T* b, T* direction, T* next,
                             T previous_factor, T residual_factor, int first);
-// Fine x, b in layout hx, coarse b, x in layout hxc.
+// What the producer of a level's rhs b writes to its x: zero, or the first
+// pre-smoothing step from x = 0, which needs no neighbour (the row of a zero
+// x is zero): the first Chebyshev stage x = factor * b / D (also the stage's
+// direction, written when another stage follows), or the first red-black
+// colour.  kZeroNone leaves x unwritten.
+enum ZeroKind : int { kZeroClear = 0, kZeroChebyshev = 1, kZeroRedBlack = 2, kZeroNone = 3 };
+template <class T>
+struct ZeroStart {
+  int kind;
+  T factor;
+  const T* diag;   // the level's, natural order
+  T* direction;    // null when no further Chebyshev stage follows
+};
+// Fine x, b in layout hx, coarse b, x in layout hxc (zero: point levels, natural order).
 template <class T>
 void launch_defect_restrict(cudaStream_t s, const Level<T>& F, const T* x,
                             const T* b, const Level<T>& C, T* cb, T* cx,
-                            int coarsen_mask, int hx = 0, int hxc = 0);
+                            int coarsen_mask, int hx, int hxc, const ZeroStart<T>& zero);
 // Fine x in layout hx, coarse x in layout hxc.
 template <class T>
 void launch_prolongate(cudaStream_t s, const Level<T>& F, T* x,
@@ -199,12 +212,65 @@ int tail_grid(int steps, int dense_n, int sms);
 template <class T>
 bool launch_tail(cudaStream_t s, const TailProgram<T>& prog, int steps, int blocks);
 
+// ---- the smallest point levels as one launch (kernels_small.cu) -------------
+// Levels of a point-smoothed hierarchy with at most kSmallMaxCells cells, from
+// the first such level to the coarsest.  One CTA runs them: measured at 64^3
+// (FP64 MG application, levels 8^3 and below; with the first smoothing step
+// folded into the producers of the rhs) 357 -> 223 us.  At 16^3 a stage reads
+// its coefficients at one SM's rate, no faster than a launch of 16 CTAs.
+constexpr int kSmallMaxCells = 1023;
+constexpr int kSmallMaxLevels = 12;
+constexpr int kSmallMaxOps = 1024;
+constexpr int kSmallMaxStages = 16;
+constexpr size_t kSmallMaxShared = 200 * 1024;
+enum SmallKind : int {
+  kSmallStage = 0,    // Chebyshev stage `arg`
+  kSmallColour = 1,   // red-black colour `arg`
+  kSmallDefect = 2,   // defect into vector R
+  kSmallGather = 3,   // rhs from the finer level's defects, x by ZeroKind `arg`
+  kSmallStart = 4,    // x by ZeroKind `arg` from the level's own rhs
+  kSmallProlong = 5,  // add the next level's vector `arg`
+  kSmallCoarse = 6    // all sweeps of the coarsest level
+};
+// Vectors of a level: two x (a Chebyshev stage writes the other one), b, and
+// the direction or defect.
+enum SmallVector : int { kSmallX = 0, kSmallX2 = 1, kSmallB = 2, kSmallR = 3, kSmallVectors = 4 };
+template <class T>
+struct SmallLevel {
+  Level<T> view;
+  int mask;           // axes that coarsen to the next level
+  int coefficients, cells, vectors;  // byte offsets in shared memory
+};
+template <class T>
+struct SmallProgram {
+  int count;          // levels
+  int ops;
+  int coarse_sweeps;
+  int result;         // x vector of the first level that holds the result
+  int wide;           // byte offset of the coarsest level's FP64 copies
+  const T* b;         // first level's rhs
+  T* x;               // and result
+  Level<double> coarse;
+  T previous_factor[kSmallMaxStages];
+  T residual_factor[kSmallMaxStages];
+  SmallLevel<T> level[kSmallMaxLevels];
+  // kind | level << 4 | arg << 8 | current x vector << 16
+  unsigned op[kSmallMaxOps];
+};
+static_assert(sizeof(SmallProgram<double>) < 32000, "kernel parameter limit");
+// Lays the program out in shared memory and returns the bytes it takes.
+template <class T>
+size_t small_layout(SmallProgram<T>& prog);
+// False (nothing launched) when it takes more than kSmallMaxShared.
+template <class T>
+bool launch_small_cycle(cudaStream_t s, SmallProgram<T>& prog);
+
 // ---- MG entry/exit ------------------------------------------------------
-// b = active ? r : 0 (converted to T), and x = 0 when zero_x; b and x in
-// layout v, r natural.
+// b = active ? r : 0 (converted to T), and x by `zero` (its Chebyshev and
+// red-black starts only in natural order); b and x in layout v, r natural.
 template <class T>
 void launch_mg_enter(cudaStream_t s, int n, const double* r,
-                     const uint8_t* active, T* b, T* x, VecLayout v, bool zero_x);
+                     const uint8_t* active, T* b, T* x, VecLayout v, const ZeroStart<T>& zero);
 // z = active ? x * scale : 0 (scale read from device when scale_ptr).
 template <class T>
 void launch_mg_exit(cudaStream_t s, int n, const T* x, const uint8_t* active,

@@ -205,6 +205,21 @@ __device__ __forceinline__ void chebyshev_cell(const Level<T>& L, const T* x, co
   next[c] = Ld::get(x + c) + d;
 }
 
+// x of one cell after the start from x = 0 (ZeroKind `kind`): `d` gets the
+// first Chebyshev direction.  The row of a zero x is an exact zero, so the
+// arithmetic is chebyshev_cell's and rb_slot's with that value.  `parity` is
+// the cell's i + j + k modulo 2 (colour 0 goes first).
+template <class T>
+__device__ __forceinline__ T zero_start_value(int kind, T factor, T b, T diag, int parity, T& d) {
+  d = T(0);
+  if (kind == 1) {
+    d = factor * b / diag;
+    return T(0) + d;
+  }
+  if (kind == 2 && parity == 0) return T(0) + T(0.72) * b / diag;
+  return T(0);
+}
+
 // ---------------------------------------------------------------------------
 // Transfers (kernels.cu).
 
@@ -268,16 +283,13 @@ __device__ __forceinline__ void interp_axis(int fine, int coarsened,
 // LdC reads the coarse correction, which is stored in layout CPos; the
 // cell's x sits at x[at].
 // MASK >= 0 fixes the coarsening mask at compile time, so the terms of an
-// axis that is not coarsened (and their loads) drop out.
-template <class T, class Ld = PlainLoad, class LdC = PlainLoad, int MASK = -1,
-          class CPos = NaturalPos>
-__device__ __forceinline__ T prolongate_cell(const Level<T>& F, const T* x, const Level<T>& C,
-                                             const T* cx, int mask, int c, int i, int j, int k,
-                                             int at, CPos cpos = CPos()) {
+// axis that is not coarsened (and their loads) drop out.  prolongate_at is
+// the interpolated correction alone.
+template <class T, class LdC = PlainLoad, int MASK = -1, class CPos = NaturalPos>
+__device__ __forceinline__ T prolongate_at(const Level<T>& C, const T* cx, int mask, int i, int j,
+                                           int k, CPos cpos) {
   const int m = MASK >= 0 ? MASK : mask;
   const int mx = m & 1, my = (m >> 1) & 1, mz = (m >> 2) & 1;
-  const bool fluid = F.fluid[c] != 0;
-  const T old = Ld::get(x + at);
   int xi[2], yi[2], zi[2];
   double xw, yw, zw;
   interp_axis(i, mx, C.nx, xi[0], xi[1], xw);
@@ -310,6 +322,17 @@ __device__ __forceinline__ T prolongate_cell(const Level<T>& F, const T* x, cons
         const T sum = value + term[az][ay][ax];
         value = on ? sum : value;
       }
+  return value;
+}
+
+template <class T, class Ld = PlainLoad, class LdC = PlainLoad, int MASK = -1,
+          class CPos = NaturalPos>
+__device__ __forceinline__ T prolongate_cell(const Level<T>& F, const T* x, const Level<T>& C,
+                                             const T* cx, int mask, int c, int i, int j, int k,
+                                             int at, CPos cpos = CPos()) {
+  const bool fluid = F.fluid[c] != 0;
+  const T old = Ld::get(x + at);
+  const T value = prolongate_at<T, LdC, MASK, CPos>(C, cx, mask, i, j, k, cpos);
   return fluid ? old + value : T(0);
 }
 

@@ -411,6 +411,7 @@ Status Solver::allocate() {
       b.lfac[ax] = reinterpret_cast<float*>(at(o.lf32[ax]));
     }
   }
+  select_small();
   return check(cudaStreamSynchronize(stream_), "allocation");
 }
 
@@ -713,28 +714,66 @@ Status Solver::correct_flux(const double* correction, const double* cx, const do
 // ---------------------------------------------------------------------------
 // MG cycle (mg_cycle, src/solver_mg.cpp:4192-4338).
 
-// x_zero: the level's x is zero on entry (a cycle's first visit), which the
-// chunked scan uses to skip reading it in the first sweep.
+namespace {
+// Factors of Chebyshev stage s = 0, 1, ... (chebyshev_point_smooth_streamed,
+// src/solver_mg.cpp:2916-3012).
+struct ChebyshevStages {
+  double theta, delta, sigma, previous_rho;
+  int s{0};
+  explicit ChebyshevStages(double lower_fraction) {
+    constexpr double beta = 2.0;
+    const double alpha = lower_fraction * beta;
+    theta = (beta + alpha) * 0.5;
+    delta = (beta - alpha) * 0.5;
+    sigma = theta / delta;
+    previous_rho = 1.0 / sigma;
+  }
+  void next(double& previous_factor, double& residual_factor) {
+    const double rho = s == 0 ? 0.0 : 1.0 / (2.0 * sigma - previous_rho);
+    previous_factor = s == 0 ? 0.0 : rho * previous_rho;
+    residual_factor = s == 0 ? 1.0 / theta : 2.0 * rho / delta;
+    if (s != 0) previous_rho = rho;
+    ++s;
+  }
+};
+}  // namespace
+
+// On a point level the first pre-smoothing step from x = 0 needs no neighbour,
+// so the kernel that writes the level's rhs takes it (write_zero_start) instead
+// of clearing x; the step's own launch, its read of a zero x and of the faces
+// drop out.  The null-space projection changes the rhs after it was written,
+// so it keeps the plain start.
+template <class T>
+ZeroStart<T> Solver::zero_start(const std::vector<DeviceLevel<T>>& levels, int level) const {
+  const DeviceLevel<T>& L = levels[level];
+  if (level == small_level_) return {kZeroNone, T(0), nullptr, nullptr};
+  if (level + 1 == static_cast<int>(levels.size()) || L.line_mask != 0 ||
+      policy_.null_space != HFPS_NULL_SPACE_NONE)
+    return {kZeroClear, T(0), nullptr, nullptr};
+  if (!L.chebyshev) return {kZeroRedBlack, T(0), L.diag, nullptr};
+  double previous, residual;
+  ChebyshevStages(policy_.chebyshev_lower_spectrum_fraction).next(previous, residual);
+  return {kZeroChebyshev, static_cast<T>(residual), L.diag,
+          policy_.pre_sweeps > 1 ? L.r : nullptr};
+}
+
+// x_zero: the level's x started from zero (a cycle's first visit).  On point
+// levels its first step is then already taken (zero_start); the chunked scan
+// uses it to skip reading x in the first sweep.
 template <class T>
 void Solver::smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
                     bool reverse, bool x_zero) {
   DeviceLevel<T>& L = levels[level];
   const Level<T> view = L.view(neumann_);
   if (L.line_mask == 0) {
+    const bool started = x_zero && policy_.null_space == HFPS_NULL_SPACE_NONE;
     if (L.chebyshev) {
-      // chebyshev_point_smooth_streamed (src/solver_mg.cpp:2916-3012): the
-      // ping-pong partner becomes the solution after odd stage counts.
-      constexpr double beta = 2.0;
-      const double alpha = policy_.chebyshev_lower_spectrum_fraction * beta;
-      const double theta = (beta + alpha) * 0.5;
-      const double delta = (beta - alpha) * 0.5;
-      const double sigma = theta / delta;
-      double previous_rho = 1.0 / sigma;
+      // The ping-pong partner becomes the solution after odd stage counts.
+      ChebyshevStages stages(policy_.chebyshev_lower_spectrum_fraction);
       for (int s = 0; s < sweeps; ++s) {
-        const double rho = s == 0 ? 0.0 : 1.0 / (2.0 * sigma - previous_rho);
-        const double previous_factor = s == 0 ? 0.0 : rho * previous_rho;
-        const double residual_factor = s == 0 ? 1.0 / theta : 2.0 * rho / delta;
-        if (s != 0) previous_rho = rho;
+        double previous_factor, residual_factor;
+        stages.next(previous_factor, residual_factor);
+        if (started && s == 0) continue;
         launch_chebyshev_stage<T>(stream_, view, L.x, L.b, L.r, L.t,
                                   static_cast<T>(previous_factor),
                                   static_cast<T>(residual_factor), s == 0 ? 1 : 0);
@@ -743,8 +782,10 @@ void Solver::smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
     } else {
       const int first = reverse ? 1 : 0;
       for (int s = 0; s < sweeps; ++s)
-        for (int pass = 0; pass < 2; ++pass)
+        for (int pass = 0; pass < 2; ++pass) {
+          if (started && s == 0 && pass == 0) continue;
           launch_rb_color<T>(stream_, view, L.x, L.b, (first + pass) & 1);
+        }
     }
     return;
   }
@@ -796,6 +837,105 @@ void Solver::coarse_solve(std::vector<DeviceLevel<T>>& levels, bool x_zero) {
       launch_coarse_solve<T, double>(stream_, view, L.x, L.b, xs, bs, D.t, D.r,
                                      policy_.coarse_sweeps, a);
   }
+}
+
+// The one-CTA launch covers the point levels from the first of at most
+// kSmallMaxCells cells whose program (shared memory, phases) fits.
+void Solver::select_small() {
+  small_level_ = -1;
+  const int levels = static_cast<int>(l64_.size());
+  if (policy_.null_space != HFPS_NULL_SPACE_NONE || policy_.pre_sweeps > kSmallMaxStages ||
+      policy_.post_sweeps > kSmallMaxStages)
+    return;
+  for (int l = 0; l < levels; ++l) {
+    if (l64_[l].line_mask != 0) return;
+    if (l64_[l].cells() > kSmallMaxCells || levels - l > kSmallMaxLevels) continue;
+    SmallProgram<double> prog;
+    if (!small_program(l64_, l, policy_.cycle == 1 ? 2 : 1, true, prog) ||
+        small_layout(prog) > kSmallMaxShared)
+      continue;
+    small_level_ = l;
+    return;
+  }
+}
+
+template <class T>
+bool Solver::small_ops(const std::vector<DeviceLevel<T>>& levels, int first, int level,
+                       int counter, bool x_zero, int* slot, SmallProgram<T>& prog) const {
+  const int l = level - first;
+  const int last = static_cast<int>(levels.size()) - 1;
+  const auto add = [&](int kind, int lv, int arg) {
+    if (prog.ops >= kSmallMaxOps) return false;
+    prog.op[prog.ops++] = static_cast<unsigned>(kind) | static_cast<unsigned>(lv) << 4 |
+                          static_cast<unsigned>(arg) << 8 |
+                          static_cast<unsigned>(slot[lv]) << 16;
+    return true;
+  };
+  if (level == last) return add(kSmallCoarse, l, 0);
+  const bool chebyshev = levels[level].chebyshev;
+  // smooth(): the first step from x = 0 is taken by the start or the gather.
+  const auto smoother = [&](int sweeps, bool reverse, bool started) {
+    bool ok = true;
+    if (chebyshev) {
+      for (int s = started ? 1 : 0; s < sweeps; ++s) {
+        ok = ok && add(kSmallStage, l, s);
+        slot[l] ^= 1;
+      }
+    } else {
+      for (int p = started ? 1 : 0; p < 2 * sweeps; ++p)
+        ok = ok && add(kSmallColour, l, (p + (reverse ? 1 : 0)) & 1);
+    }
+    return ok;
+  };
+  const int below = level + 1 == last ? kZeroClear
+                                      : (levels[level + 1].chebyshev ? kZeroChebyshev
+                                                                     : kZeroRedBlack);
+  return smoother(policy_.pre_sweeps, false, x_zero) && add(kSmallDefect, l, 0) &&
+         add(kSmallGather, l + 1, below) &&
+         small_ops(levels, first, level + 1, counter, true, slot, prog) &&
+         (counter <= 1 ||
+          small_ops(levels, first, level + 1, counter - 1, false, slot, prog)) &&
+         add(kSmallProlong, l, slot[l + 1]) && smoother(policy_.post_sweeps, true, false);
+}
+
+template <class T>
+bool Solver::small_program(const std::vector<DeviceLevel<T>>& levels, int first, int counter,
+                           bool both, SmallProgram<T>& prog) const {
+  const int count = static_cast<int>(levels.size()) - first;
+  prog.count = count;
+  prog.ops = 0;
+  prog.coarse_sweeps = policy_.coarse_sweeps;
+  prog.coarse = l64_.back().view(neumann_);
+  prog.b = levels[first].b;
+  prog.x = levels[first].x;
+  ChebyshevStages stages(policy_.chebyshev_lower_spectrum_fraction);
+  for (int s = 0; s < kSmallMaxStages; ++s) {
+    double previous, residual;
+    stages.next(previous, residual);
+    prog.previous_factor[s] = static_cast<T>(previous);
+    prog.residual_factor[s] = static_cast<T>(residual);
+  }
+  int slot[kSmallMaxLevels] = {};
+  for (int l = 0; l < count; ++l) {
+    prog.level[l].view = levels[first + l].view(neumann_);
+    prog.level[l].mask = levels[first + l].coarsen_mask;
+  }
+  if (count > 1)
+    prog.op[prog.ops++] =
+        static_cast<unsigned>(kSmallStart) |
+        static_cast<unsigned>(levels[first].chebyshev ? kZeroChebyshev : kZeroRedBlack) << 8;
+  const bool ok = small_ops(levels, first, first, counter, true, slot, prog) &&
+                  (!both || counter <= 1 ||
+                   small_ops(levels, first, first, counter - 1, false, slot, prog));
+  prog.result = slot[0];
+  return ok;
+}
+
+template <class T>
+void Solver::small_cycle(std::vector<DeviceLevel<T>>& levels, int counter, bool both) {
+  SmallProgram<T> prog;
+  small_program(levels, small_level_, counter, both, prog);
+  launch_small_cycle<T>(stream_, prog);
 }
 
 // The persistent small-level launch covers levels tail_level_.. when every
@@ -914,6 +1054,10 @@ void Solver::tail_launch(std::vector<DeviceLevel<T>>& levels, TailProgram<T>& pr
 template <class T>
 void Solver::cycle(std::vector<DeviceLevel<T>>& levels, int level, int counter,
                    bool x_zero) {
+  if (level == small_level_) {  // the finest level itself; see below for the others
+    small_cycle(levels, counter, false);
+    return;
+  }
   if (level + 1 == static_cast<int>(levels.size())) {
     coarse_solve(levels, x_zero);
     return;
@@ -923,12 +1067,15 @@ void Solver::cycle(std::vector<DeviceLevel<T>>& levels, int level, int counter,
   smooth(levels, level, policy_.pre_sweeps, false, x_zero);
   // Retained defect + restrict_residual in one pass.
   launch_defect_restrict<T>(stream_, F.view(neumann_), F.x, F.b, C.view(neumann_),
-                            C.b, C.x, F.coarsen_mask, F.split, C.split);
+                            C.b, C.x, F.coarsen_mask, F.split, C.split,
+                            zero_start(levels, level + 1));
   // restrict_residual's projection of the coarse rhs (src/solver_mg.cpp:3708-3716).
   if (policy_.null_space == HFPS_NULL_SPACE_CONSTANT)
     launch_project_constant<T>(stream_, C.nx, C.ny, C.nz, C.split, C.b, volume_[level + 1],
                                d_scalars_, d_partials_);
-  if (level + 1 == tail_level_) {
+  if (level + 1 == small_level_) {
+    small_cycle(levels, counter, true);
+  } else if (level + 1 == tail_level_) {
     // Both visits of the level below (an F-cycle's counter 2 and 1) in one
     // persistent launch.
     TailProgram<T> prog;
@@ -971,8 +1118,9 @@ void Solver::mg_enqueue(std::vector<DeviceLevel<T>>& levels, const double* r,
   const VecLayout v0{L0.nx, L0.ny, L0.split};
   // x = 0 is written here unless the diagonal shortcut or the first
   // pre-smoothing sweep (zero flags) defines every entry anyway.
-  const bool zero_x = !(diagonal_shortcut_ || first_sweep_zero_);
-  launch_mg_enter<T>(stream_, n, r, d_active_, L0.b, L0.x, v0, zero_x);
+  ZeroStart<T> zero = zero_start(levels, 0);
+  if (diagonal_shortcut_ || first_sweep_zero_) zero.kind = kZeroNone;
+  launch_mg_enter<T>(stream_, n, r, d_active_, L0.b, L0.x, v0, zero);
   // MgNullSpace::constant: the rhs, every restricted rhs and the result lose
   // their volume-weighted mean (apply_impl, src/solver_mg.cpp:4900-4960).
   const bool constant = policy_.null_space == HFPS_NULL_SPACE_CONSTANT;
@@ -2203,7 +2351,8 @@ Status Solver::profile_kernel(int kernel, int repetitions, double* ms,
       case HFPS_KERNEL_RESTRICT_FP64:
         launch_defect_restrict<double>(stream_, A, L0.x, L0.b, l64_[1].view(neumann_),
                                        l64_[1].b, l64_[1].x, L0.coarsen_mask, L0.split,
-                                       l64_[1].split);
+                                       l64_[1].split,
+                                       ZeroStart<double>{kZeroClear, 0.0, nullptr, nullptr});
         per_cell = 48.0 + 2.0 * 8.0 / (l64_[0].cells() / static_cast<double>(l64_[1].cells()));
         break;
       case HFPS_KERNEL_PROLONG_FP64:

@@ -115,6 +115,22 @@ class Solver {
               bool reverse, bool x_zero);
   template <class T>
   void coarse_solve(std::vector<DeviceLevel<T>>& levels, bool x_zero);
+  // What the producer of `level`'s rhs writes to its x (ZeroKind).
+  template <class T>
+  ZeroStart<T> zero_start(const std::vector<DeviceLevel<T>>& levels, int level) const;
+  // The smallest point levels as one launch: small_ops appends the phases of
+  // cycle(level, counter), false when they do not fit; small_program builds
+  // the program of consecutive visits of the first such level with the given
+  // counters, and small_cycle launches it.
+  void select_small();
+  template <class T>
+  bool small_ops(const std::vector<DeviceLevel<T>>& levels, int first, int level, int counter,
+                 bool x_zero, int* slot, SmallProgram<T>& prog) const;
+  template <class T>
+  bool small_program(const std::vector<DeviceLevel<T>>& levels, int first, int counter,
+                     bool both, SmallProgram<T>& prog) const;
+  template <class T>
+  void small_cycle(std::vector<DeviceLevel<T>>& levels, int counter, bool both);
   // The small levels as one persistent launch: tail_cycle appends the
   // phases of cycle(level, counter) to `prog` exactly as cycle() would
   // launch them (same buffer roles and swaps); tail_launch runs a program.
@@ -184,6 +200,8 @@ class Solver {
   double* coarse_op_{};
   int coarse_axis_{-1};
   bool coarse_dense_{};
+  // First level of the one-CTA launch of the smallest point levels (-1: none).
+  int small_level_{-1};
   // First level of the persistent small-level launch (-1: every phase is
   // its own kernel), its PCR width and co-resident grid per precision.
   int tail_level_{-1};
