@@ -216,11 +216,17 @@ constexpr int kScanMaxExtent =
         ? HFPS_SCAN_ROWS_F64 * HFPS_SCAN_THREADS_F64
         : HFPS_SCAN_ROWS_F32 * HFPS_SCAN_THREADS_F32;
 
+//
+// x-lines (k_line_scan_x) keep a line's rows together instead, as their
+// vectors do: ((e * 2 + colour) * colour_lines + t) * extent + s.
 struct ScanLayout {
   int extent;
   int colour_lines;
+  bool rows_together;
   __host__ __device__ size_t cell(int e, int colour, int s, int t) const {
-    return ((static_cast<size_t>(e) * 2 + colour) * extent + s) * colour_lines + t;
+    const size_t block = (static_cast<size_t>(e) * 2 + colour);
+    return rows_together ? (block * colour_lines + t) * extent + s
+                         : (block * extent + s) * colour_lines + t;
   }
   __host__ __device__ size_t values(int arrays) const {
     return static_cast<size_t>(arrays) * 2 * extent * colour_lines;
@@ -236,7 +242,7 @@ __global__ void k_scan_factors(Level<T> L, int axis, T* __restrict__ fac) {
   const int lines = a_extent * b_extent;
   const int extent = line_extent(axis, L.nx, L.ny, L.nz);
   const int ha = (a_extent + 1) >> 1;
-  const ScanLayout lay{extent, ha * b_extent};
+  const ScanLayout lay{extent, ha * b_extent, axis == 0};
   for (int line = blockIdx.x * blockDim.x + threadIdx.x; line < lines;
        line += gridDim.x * blockDim.x) {
     const int fb = line / a_extent;
@@ -286,7 +292,7 @@ __global__ void __launch_bounds__(ScanConfig<T>::threads)
   const int a_extent = AXIS == 0 ? L.ny : L.nx;
   const int b_extent = AXIS == 2 ? L.ny : L.nz;
   const int ha = (a_extent + 1) >> 1;
-  const ScanLayout lay{extent, ha * b_extent};
+  const ScanLayout lay{extent, ha * b_extent, false};
   const int lane = threadIdx.x;
   const int q = threadIdx.y;
   const int t = blockIdx.x * LPB + lane;
@@ -380,6 +386,182 @@ __global__ void __launch_bounds__(ScanConfig<T>::threads)
     const T xv = v[u] - __ldg(uf + srow(u) * row) * xn;
     xn = u < rows ? xv : xn;
     if (u < rows) x[base + srow(u) * stride] = xn;
+  }
+}
+
+// The same colour pass for x-lines, whose rows are contiguous.  Lanes across
+// lines would touch a 32-byte sector per value (the pass took 155 us on
+// 456x256x52 in FP64, 1.4 TB/s), so here a warp walks each line along its
+// rows: the right-hand sides are formed coalesced and left in shared memory,
+// the factors follow by asynchronous copies that hold no registers, each
+// thread then scans its chunk of up to ScanConfig<T>::rows rows out of shared
+// memory (chunks padded to an odd length, so that the lanes of a line fall in
+// different banks), and the solution goes back coalesced: 83 us, 2.6 TB/s of
+// the 36 bytes per cell that a pass needs (the transverse faces are 16 of them,
+// the factors 8).  A block of at most 2048 rows takes 52 KB of shared memory,
+// so that four blocks per SM overlap their load and scan phases; what bounds
+// it now is the rest of that overlap.  Chunks, compositions and their
+// order are k_line_scan_color's, so the results are bit for bit its results.
+constexpr int kScanXThreads = 128;
+
+template <class T>
+__device__ __forceinline__ void copy_async(T* shared, const T* global) {
+  const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(shared));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(global),
+               "n"(sizeof(T)));
+}
+
+struct ScanXShape {
+  int lines;        // per block
+  int chunks, rows; // per line, per chunk
+  int pitch;        // shared-memory stride of a chunk
+};
+
+template <class T>
+__global__ void __launch_bounds__(kScanXThreads * (sizeof(T) == 4 ? 2 : 1))
+    k_line_scan_x(Level<T> L, T* x, const T* __restrict__ rhs, const T* __restrict__ fac,
+                  int color, ScanXShape sh) {
+  grid_dependency_sync();
+  extern __shared__ unsigned char scan_x_smem[];
+  constexpr bool kSym = ScanConfig<T>::symmetric;
+  constexpr int kScanRows = ScanConfig<T>::rows;
+  const int extent = L.nx;
+  const int ha = (L.ny + 1) >> 1;
+  const ScanLayout lay{extent, ha * L.nz, true};
+  const int m = sh.rows, S = sh.chunks;
+  const int line_pitch = S * sh.pitch;
+  const int span = sh.lines * line_pitch;
+  T* d = reinterpret_cast<T*>(scan_x_smem);
+  T* inv = d + span;
+  T* up = inv + span;
+  T* low = kSym ? up : up + span;
+  T* fA = low + span;
+  T* fB = fA + sh.lines * S;
+  T* bA = fB + sh.lines * S;
+  T* bB = bA + sh.lines * S;
+  // s / m for s < 2048 and m <= 16.
+  const unsigned reciprocal = (65536u + m - 1) / m;
+  const auto place = [&](int s) {
+    const int q = static_cast<int>((static_cast<unsigned>(s) * reciprocal) >> 16);
+    return q * sh.pitch + (s - q * m);
+  };
+  const int t0 = blockIdx.x * sh.lines;
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+  // A line's index in its colour, or false past the colour's lines.
+  const auto locate = [&](int t, int& fa, int& fb) {
+    fb = t / ha;
+    fa = 2 * (t - fb * ha) + ((fb + color) & 1);
+    return t < ha * L.nz && fa < L.ny;
+  };
+  for (int l = warp; l < sh.lines; l += warps) {
+    int fa, fb;
+    if (!locate(t0 + l, fa, fb)) continue;
+    const T* finv = fac + lay.cell(0, color, 0, t0 + l);
+    const T* flow = fac + lay.cell(1, color, 0, t0 + l);
+    const T* fup = fac + lay.cell(kSym ? 1 : 2, color, 0, t0 + l);
+    for (int s = lane; s < extent; s += 32) {
+      const int at = l * line_pitch + place(s);
+      copy_async(inv + at, finv + s);
+      copy_async(up + at, fup + s);
+      if constexpr (!kSym) copy_async(low + at, flow + s);
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int l = warp; l < sh.lines; l += warps) {
+    int fa, fb;
+    if (!locate(t0 + l, fa, fb)) continue;
+    const LineRhs<T, 0, false> lr(L, fa, fb, 0);
+    const int base = L.nx * (fa + L.ny * fb);
+#pragma unroll 4
+    for (int s = lane; s < extent; s += 32) {
+      const int c = base + s;
+      T v = __ldg(rhs + c);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const int f = lr.fbase[n] + s * lr.fstride[n];
+        const T lo = __ldg(x + c + lr.off[2 * n]);
+        const T hi = __ldg(x + c + lr.off[2 * n + 1]);
+        v += __ldg(lr.face[n] + f) * (lr.keep[2 * n] ? lo : T(0));
+        v += __ldg(lr.face[n] + f + lr.fhigh[n]) * (lr.keep[2 * n + 1] ? hi : T(0));
+      }
+      if (s == 0) v += lr.end_low * (lr.lkeep_low ? x[c] : T(0));
+      if (s + 1 == extent) v += lr.end_high * (lr.lkeep_high ? x[c] : T(0));
+      d[l * line_pitch + place(s)] = v;
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  const int l = threadIdx.x / S, q = threadIdx.x - l * S;
+  int fa, fb;
+  const bool valid = l < sh.lines && locate(t0 + l, fa, fb);
+  const int rows = valid ? max(0, min(m, extent - q * m)) : 0;
+  const int at = valid ? l * line_pitch + q * sh.pitch : 0;
+  const int slot = valid ? l * S + q : 0;
+  // Forward multiplier of row u of the chunk: u_{s-1} (zero on row 0), or l_s.
+  const auto lower = [&](int u) -> T {
+    if constexpr (kSym) {
+      if (u > 0) return up[at + u - 1];
+      return q > 0 ? up[at - sh.pitch + m - 1] : T(0);
+    } else {
+      return low[at + u];
+    }
+  };
+  T v[kScanRows];
+  T A = T(1), B = T(0);
+#pragma unroll
+  for (int u = 0; u < kScanRows; ++u) {
+    if (u < rows) {
+      v[u] = d[at + u];
+      if constexpr (!kSym) v[u] = v[u] * inv[at + u];
+      const T f = lower(u);
+      B = v[u] - f * B;
+      A = -f * A;
+    }
+  }
+  if (valid) {
+    fA[slot] = A;
+    fB[slot] = B;
+  }
+  __syncthreads();
+  T z = T(0);
+  for (int p = 0; p < q; ++p) z = valid ? fA[slot - q + p] * z + fB[slot - q + p] : T(0);
+#pragma unroll
+  for (int u = 0; u < kScanRows; ++u) {
+    if (u < rows) {
+      z = v[u] - lower(u) * z;
+      if constexpr (kSym) v[u] = z * inv[at + u];
+      else v[u] = z;
+    }
+  }
+  A = T(1);
+  B = T(0);
+#pragma unroll
+  for (int u = kScanRows - 1; u >= 0; --u) {
+    if (u < rows) {
+      const T f = up[at + u];
+      B = v[u] - f * B;
+      A = -f * A;
+    }
+  }
+  if (valid) {
+    bA[slot] = A;
+    bB[slot] = B;
+  }
+  __syncthreads();
+  T xn = T(0);
+  for (int p = S - 1; p > q; --p) xn = valid ? bA[slot - q + p] * xn + bB[slot - q + p] : T(0);
+#pragma unroll
+  for (int u = kScanRows - 1; u >= 0; --u) {
+    if (u < rows) {
+      xn = v[u] - up[at + u] * xn;
+      d[at + u] = xn;
+    }
+  }
+  __syncthreads();
+  for (int k = warp; k < sh.lines; k += warps) {
+    if (!locate(t0 + k, fa, fb)) continue;
+    T* out = x + L.nx * (fa + L.ny * fb);
+    for (int s = lane; s < extent; s += 32) out[s] = d[k * line_pitch + place(s)];
   }
 }
 
@@ -618,18 +800,13 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
                  int color, long long per_color, const ScanShape& sh, ScanFlags f) {
   const int blocks = static_cast<int>((per_color + LPB - 1) / LPB);
   const size_t smem = static_cast<size_t>(4) * sh.chunks * LPB * sizeof(T);
-  // The zero variants and split rows only on y- and z-line levels (x-line
-  // levels keep the natural order and always read x, which the cycle has
-  // cleared).
   const dim3 block(LPB, sh.chunks);
-  constexpr bool kYZ = AXIS != 0;
-  const int mode = !kYZ ? kScanNormal
-                        : (f.zero_other && f.zero_self ? kScanFresh
-                                                       : (f.zero_self ? kScanOwnZero : kScanNormal));
-  const bool split = kYZ && f.hx != 0;
-#define HFPS_SCAN_LAUNCH(MODE, SPLIT)                                                         \
-  launch(k_line_scan_color<T, AXIS, LPB, kYZ ? MODE : kScanNormal, kYZ && SPLIT>, blocks, block, \
-         smem, s, L, x, b, fac, color, sh.rows, f.hx)
+  const int mode = f.zero_other && f.zero_self ? kScanFresh
+                                               : (f.zero_self ? kScanOwnZero : kScanNormal);
+  const bool split = f.hx != 0;
+#define HFPS_SCAN_LAUNCH(MODE, SPLIT)                                                       \
+  launch(k_line_scan_color<T, AXIS, LPB, MODE, SPLIT>, blocks, block, smem, s, L, x, b, fac, \
+         color, sh.rows, f.hx)
   if (mode == kScanFresh) {
     if (split) HFPS_SCAN_LAUNCH(kScanFresh, true);
     else HFPS_SCAN_LAUNCH(kScanFresh, false);
@@ -641,6 +818,27 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
     else HFPS_SCAN_LAUNCH(kScanNormal, false);
   }
 #undef HFPS_SCAN_LAUNCH
+}
+
+// As many lines per block as its threads have chunks for.
+template <class T>
+void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* fac, int color,
+                   long long per_color) {
+  constexpr int rows = ScanConfig<T>::rows;
+  constexpr int threads = kScanXThreads * (sizeof(T) == 4 ? 2 : 1);
+  ScanXShape sh{};
+  sh.chunks = (L.nx + rows - 1) / rows;
+  sh.rows = (L.nx + sh.chunks - 1) / sh.chunks;
+  sh.pitch = sh.rows | 1;
+  sh.lines = threads / sh.chunks;
+  const int arrays = 1 + ScanConfig<T>::arrays;
+  const size_t smem = static_cast<size_t>(sh.lines) * sh.chunks *
+                      (static_cast<size_t>(arrays) * sh.pitch + 4) * sizeof(T);
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(k_line_scan_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(smem));
+  launch(k_line_scan_x<T>, static_cast<int>((per_color + sh.lines - 1) / sh.lines), threads, smem,
+         s, L, x, b, fac, color, sh);
 }
 
 template <class T, int AXIS>
@@ -678,7 +876,7 @@ size_t line_factor_values(int nx, int ny, int nz, int axis) {
   const int kind = line_kind(nx, ny, nz, axis);
   if (kind == kLineNone) return 0;
   if (kind == kLineScan)
-    return ScanLayout{extent, ((a_extent + 1) / 2) * b_extent}.values(ScanConfig<T>::arrays);
+    return ScanLayout{extent, ((a_extent + 1) / 2) * b_extent, axis == 0}.values(ScanConfig<T>::arrays);
   int P, lpb, steps;
   pcr_shape(extent, P, lpb, steps);
   return static_cast<size_t>(2 * steps + 1) * lines * P;
@@ -714,10 +912,13 @@ void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
   const int kind = line_kind(L.nx, L.ny, L.nz, axis);
   if (kind == kLineNone) return;
   if (kind == kLineScan) {
+    if (axis == 0) {
+      launch_scan_x<T>(s, L, x, b, fac, color, per_color);
+      return;
+    }
     const ScanShape sh = scan_shape<T>(per_color, extent);
-    const ScanFlags f{axis == 0 ? 0 : hx, zero_other, zero_self};
-    if (axis == 0) launch_scan_axis<T, 0>(s, L, x, b, fac, color, per_color, sh, f);
-    else if (axis == 1) launch_scan_axis<T, 1>(s, L, x, b, fac, color, per_color, sh, f);
+    const ScanFlags f{hx, zero_other, zero_self};
+    if (axis == 1) launch_scan_axis<T, 1>(s, L, x, b, fac, color, per_color, sh, f);
     else launch_scan_axis<T, 2>(s, L, x, b, fac, color, per_color, sh, f);
     return;
   }
