@@ -147,12 +147,15 @@ void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
                       const T* fac, T* scratch, int axis, int color, int hx = 0,
                       bool zero_other = false, bool zero_self = false);
 // Coarsest level in line mode with x/rhs resident in shared memory; returns
-// false when the level is too large for that form.  With `columns`, launches
-// 2n blocks that write the columns of the sweeps' affine map x_out = P x_in
-// + M b (P then M, column-major) to x, n = cells of the level.
+// false when the level is too large for that form.  With kCoarseColumns,
+// launches 2n blocks that write the columns of the sweeps' affine map x_out =
+// P x_in + M b (P then M, column-major) to x, n = cells of the level;
+// kCoarseColumnsOn applies the sweeps to columns already there (a further
+// axis after the first).
+enum CoarseColumns : int { kCoarseVector = 0, kCoarseColumns = 1, kCoarseColumnsOn = 2 };
 template <class T, class TC>
 bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
-                        const TC* fac, int sweeps, int axis, bool columns = false);
+                        const TC* fac, int sweeps, int axis, int columns = kCoarseVector);
 // out = P x + M b with the dense coarsest-level map built by the columns
 // mode above (n <= kCoarseDenseMaxCells; out must not alias x or b).  With
 // x_zero (x is known to be zero) the P half is not read.
@@ -212,16 +215,23 @@ int tail_grid(int steps, int dense_n, int sms);
 template <class T>
 bool launch_tail(cudaStream_t s, const TailProgram<T>& prog, int steps, int blocks);
 
-// ---- the smallest point levels as one launch (kernels_small.cu) -------------
-// Levels of a point-smoothed hierarchy with at most kSmallMaxCells cells, from
-// the first such level to the coarsest.  One CTA runs them: measured at 64^3
+// ---- the smallest levels as one launch (kernels_small.cu) -------------------
+// Levels with at most kSmallMaxCells cells (and, where lines are relaxed, lines
+// of at most 2^kSmallMaxSteps cells), from the first such level to the coarsest.  One CTA runs them: measured at 64^3
 // (FP64 MG application, levels 8^3 and below; with the first smoothing step
 // folded into the producers of the rhs) 357 -> 223 us.  At 16^3 a stage reads
 // its coefficients at one SM's rate, no faster than a launch of 16 CTAs.
+// The dense map of a line hierarchy's coarsest level reads 16 n^2 bytes in
+// batches of L2 latency: with 180 rows in one CTA it took 15 us, against 4 us
+// spread over several (k_coarse_dense), so such hierarchies keep that kernel
+// and all their launches; with two strong axes (456x256x52, 8 rows, 24 sweeps
+// along both axes before) one MG application went from 4.2 to 2.9 ms.
 constexpr int kSmallMaxCells = 1023;
 constexpr int kSmallMaxLevels = 12;
 constexpr int kSmallMaxOps = 1024;
 constexpr int kSmallMaxStages = 16;
+constexpr int kSmallMaxSteps = 5;      // PCR steps of a line within a warp
+constexpr int kSmallDenseCells = 64;  // rows of the coarsest dense map (below)
 constexpr size_t kSmallMaxShared = 200 * 1024;
 enum SmallKind : int {
   kSmallStage = 0,    // Chebyshev stage `arg`
@@ -230,7 +240,9 @@ enum SmallKind : int {
   kSmallGather = 3,   // rhs from the finer level's defects, x by ZeroKind `arg`
   kSmallStart = 4,    // x by ZeroKind `arg` from the level's own rhs
   kSmallProlong = 5,  // add the next level's vector `arg`
-  kSmallCoarse = 6    // all sweeps of the coarsest level
+  kSmallCoarse = 6,   // all red-black sweeps of the coarsest level
+  kSmallLine = 7,     // line colour pass: axis | colour << 2 | PCR steps << 3
+  kSmallDense = 8     // all line sweeps of the coarsest level; 1: x is zero
 };
 // Vectors of a level: two x (a Chebyshev stage writes the other one), b, and
 // the direction or defect.
@@ -238,6 +250,7 @@ enum SmallVector : int { kSmallX = 0, kSmallX2 = 1, kSmallB = 2, kSmallR = 3, kS
 template <class T>
 struct SmallLevel {
   Level<T> view;
+  const T* factors[3];  // PCR factors per strong axis
   int mask;           // axes that coarsen to the next level
   int coefficients, cells, vectors;  // byte offsets in shared memory
 };
@@ -251,6 +264,7 @@ struct SmallProgram {
   const T* b;         // first level's rhs
   T* x;               // and result
   Level<double> coarse;
+  const double* dense;  // coarsest affine map of line levels
   T previous_factor[kSmallMaxStages];
   T residual_factor[kSmallMaxStages];
   SmallLevel<T> level[kSmallMaxLevels];

@@ -667,15 +667,16 @@ __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
 // in shared memory (widened to TC).  When each colour's lines fit the CTA's
 // thread rows, both colours' PCR factors stay in registers for all sweeps.
 //
-// With `columns` set, block j instead starts from unit data, x = e_j and
+// With kCoarseColumns, block j instead starts from unit data, x = e_j and
 // b = 0 for j < n, x = 0 and b = e_{j-n} for j >= n, and writes its result
 // to x + j*n: the columns of the affine map x_out = P x_in + M b that the
-// sweeps apply (coarse_dense_operator).
+// sweeps apply (coarse_dense_operator).  kCoarseColumnsOn starts from the
+// column that is there, with the same b.
 template <class T, class TC, int STEPS>
 __global__ void __launch_bounds__(512)
     k_coarse_line_smem(Level<TC> L, T* __restrict__ x, const T* __restrict__ b,
                        const TC* __restrict__ fac, int sweeps, int axis,
-                       bool columns) {
+                       int columns) {
   grid_dependency_sync();
   constexpr int P = 1 << STEPS;
   extern __shared__ unsigned char coarse_smem[];
@@ -685,13 +686,14 @@ __global__ void __launch_bounds__(512)
   TC* sd = bs + n + threadIdx.y * P;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   const int nthreads = blockDim.x * blockDim.y;
-  if (columns) {
+  if (columns != kCoarseVector) {
     const int j = blockIdx.x;
+    x += static_cast<size_t>(j) * n;
     for (int c = tid; c < n; c += nthreads) {
-      xs[c] = (j < n && c == j) ? TC(1) : TC(0);
+      xs[c] = columns == kCoarseColumnsOn ? static_cast<TC>(x[c])
+                                          : ((j < n && c == j) ? TC(1) : TC(0));
       bs[c] = (j >= n && c == j - n) ? TC(1) : TC(0);
     }
-    x += static_cast<size_t>(j) * n;
   } else {
     for (int c = tid; c < n; c += nthreads) {
       xs[c] = static_cast<TC>(x[c]);
@@ -943,7 +945,7 @@ void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
 
 template <class T, class TC>
 bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
-                        const TC* fac, int sweeps, int axis, bool columns) {
+                        const TC* fac, int sweeps, int axis, int columns) {
   const int extent = line_extent(axis, L.nx, L.ny, L.nz);
   if (line_kind(L.nx, L.ny, L.nz, axis) != kLinePcr) return false;
   int P, lpb, steps;
@@ -963,8 +965,9 @@ bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
       cudaFuncSetAttribute(k_coarse_line_smem<T, TC, N>,                         \
                            cudaFuncAttributeMaxDynamicSharedMemorySize,          \
                            static_cast<int>(smem));                              \
-    launch(k_coarse_line_smem<T, TC, N>, columns ? 2 * static_cast<int>(cells) : 1, block, smem, \
-                                    s, L, x, b, fac, sweeps, axis, columns);       \
+    launch(k_coarse_line_smem<T, TC, N>,                                          \
+           columns != kCoarseVector ? 2 * static_cast<int>(cells) : 1, block, smem, s, L, x, \
+           b, fac, sweeps, axis, columns);                                         \
     break;
     HFPS_COARSE_CASE(0) HFPS_COARSE_CASE(1) HFPS_COARSE_CASE(2) HFPS_COARSE_CASE(3)
     HFPS_COARSE_CASE(4) HFPS_COARSE_CASE(5) HFPS_COARSE_CASE(6) HFPS_COARSE_CASE(7)
@@ -985,9 +988,9 @@ template void launch_line_pass<double>(cudaStream_t, const Level<double>&, doubl
 template void launch_line_pass<float>(cudaStream_t, const Level<float>&, float*, const float*,
                                       const float*, float*, int, int, int, bool, bool);
 template bool launch_coarse_line<double, double>(cudaStream_t, const Level<double>&, double*,
-                                                 const double*, const double*, int, int, bool);
+                                                 const double*, const double*, int, int, int);
 template bool launch_coarse_line<float, double>(cudaStream_t, const Level<double>&, float*,
-                                                const float*, const double*, int, int, bool);
+                                                const float*, const double*, int, int, int);
 
 // ---------------------------------------------------------------------------
 // Coarsest level as a dense affine map: out = P x + M b, with P and M

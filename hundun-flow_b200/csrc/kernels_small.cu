@@ -1,4 +1,4 @@
-// The smallest point-smoothed levels of a cycle as one launch.
+// The smallest levels of a cycle as one launch.
 //
 // Below about a thousand cells a phase of the cycle (a Chebyshev stage, a
 // colour pass, a transfer) is under a microsecond of work, but as a kernel
@@ -10,7 +10,9 @@
 // and runs the whole sub-cycle (both visits of an F-cycle, which follow one
 // another) from a list of phases built on the host, with a CTA barrier
 // between phases.  The coarsest sweeps run in one warp, a cell per lane, the
-// neighbours exchanged by shuffles and nothing but registers touched.
+// neighbours exchanged by shuffles and nothing but registers touched.  Line
+// levels with lines of at most 32 cells run their colour passes as PCR within
+// a warp, and their coarsest sweeps as the dense affine map.
 //
 // What bounds it: latency.  A phase is one round of shared-memory loads, the
 // row's chain of seven dependent operations and a division, and a barrier;
@@ -18,8 +20,8 @@
 // because a phase of a thousand cells is shorter than any wait between CTAs.
 //
 // Every cell update is the one of the per-kernel path, operation for
-// operation (row_value, prolongate_at, the same stage formulas), so results
-// are bit-identical to it.
+// operation (row_value, prolongate_at, the same stage formulas, PCR), so results
+// are bit-identical to it; only the dense map groups its sums differently.
 #include "kernels.hpp"
 #include "phase_device.cuh"
 
@@ -85,6 +87,89 @@ __device__ __forceinline__ void small_coarse_warp(const Level<double>& L, T* x, 
     }
   }
   if (on) x[c] = static_cast<T>(xc);
+}
+
+// One zebra colour of line relaxation along `axis` (lines of at most 32 cells):
+// P = 2^steps lanes hold a line, its PCR steps exchange by shuffles
+// (pcr_line_slot's arithmetic, without its barriers).
+template <class T>
+__device__ __forceinline__ void small_line_pass(const Level<T>& L, T* x, const T* b,
+                                                const T* __restrict__ fac, int axis, int steps,
+                                                int color) {
+  const int P = 1 << steps;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int a_extent = axis == 0 ? L.ny : L.nx;
+  const int b_extent = axis == 2 ? L.ny : L.nz;
+  const int ha = (a_extent + 1) >> 1;
+  const int lines = ha * b_extent;
+  const int extent = line_extent(axis, L.nx, L.ny, L.nz);
+  const size_t slab = static_cast<size_t>(a_extent) * b_extent * P;
+  const int per_warp = 32 >> steps;
+  const int s = lane & (P - 1);
+  for (int t0 = warp * per_warp; t0 < lines; t0 += (kSmallThreads / 32) * per_warp) {
+    const int t = t0 + (lane >> steps);
+    const int fb = t / ha;
+    const int fa = 2 * (t - fb * ha) + ((fb + color) & 1);
+    const bool valid = t < lines && fa < a_extent;
+    const size_t at = static_cast<size_t>(valid ? fa + a_extent * fb : 0) * P + s;
+    T k[2 * kSmallMaxSteps + 1];
+#pragma unroll
+    for (int e = 0; e <= 2 * kSmallMaxSteps; ++e)
+      k[e] = e <= 2 * steps ? __ldg(fac + e * slab + at) : T(0);
+    int c = 0;
+    T d = T(0);
+    if (valid && s < extent) {
+      int i, j, m;
+      line_cell(axis, fa, fb, s, i, j, m);
+      c = i + L.nx * (j + L.ny * m);
+      d = line_rhs_any<T, PlainLoad>(L, x, b, axis, fa, fb, s, extent, c);
+    }
+    T pivot = k[0];
+#pragma unroll
+    for (int step = 0; step < kSmallMaxSteps; ++step) {
+      if (step < steps) {
+        const int h = 1 << step;
+        const T up = __shfl_up_sync(0xffffffffu, d, h);
+        const T down = __shfl_down_sync(0xffffffffu, d, h);
+        const T dlo = s - h >= 0 ? up : T(0);
+        const T dhi = s + h < P ? down : T(0);
+        d = d - dlo * k[2 * step] - dhi * k[2 * step + 1];
+        pivot = k[2 * step + 2];
+      }
+    }
+    if (valid && s < extent) x[c] = d / pivot;
+  }
+}
+
+// The coarsest sweeps as the dense affine map P x + M b (FP64, column-major,
+// P then M): groups of threads take interleaved columns of all rows, and a
+// row's partial sums are added in group order.  With x_zero the P half is not
+// read.  v holds 2n doubles, part one per thread.
+template <class T>
+__device__ __forceinline__ void small_dense(int n, const double* __restrict__ op, T* x, const T* b,
+                                            double* v, double* part, bool x_zero) {
+  const int tid = threadIdx.x;
+  for (int c = tid; c < n; c += kSmallThreads) {
+    v[c] = static_cast<double>(x[c]);
+    v[n + c] = static_cast<double>(b[c]);
+  }
+  __syncthreads();
+  const int width = (n + 31) & ~31;
+  const int groups = kSmallThreads / width;
+  const int group = tid / width, row = tid - group * width;
+  double acc = 0.0;
+  if (group < groups && row < n) {
+#pragma unroll 8
+    for (int j = (x_zero ? n : 0) + group; j < 2 * n; j += groups)
+      acc += __ldg(op + static_cast<size_t>(j) * n + row) * v[j];
+  }
+  part[tid] = acc;
+  __syncthreads();
+  if (tid < n) {
+    double sum = part[tid];
+    for (int g = 1; g < groups; ++g) sum += part[g * width + tid];
+    x[tid] = static_cast<T>(sum);
+  }
 }
 
 template <class T>
@@ -234,6 +319,14 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_cycle(const SmallProgra
         }
         break;
       }
+      case kSmallLine:
+        small_line_pass<T>(L, x, b, S.factors[arg & 3], arg & 3, arg >> 3, (arg >> 2) & 1);
+        break;
+      case kSmallDense: {
+        double* v = reinterpret_cast<double*>(smem + prog.wide);
+        small_dense<T>(n, prog.dense, x, b, v, v + 2 * n, arg != 0);
+        break;
+      }
       default: {  // kSmallCoarse
         if (n <= 32) {
           if (tid < 32) small_coarse_warp<T>(prog.coarse, x, b, prog.coarse_sweeps);
@@ -275,7 +368,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_cycle(const SmallProgra
 }  // namespace
 
 // Shared-memory layout of a program: per level the coefficients, the packed
-// cell indices and four vectors, and FP64 copies for a wide coarsest level.
+// cell indices and four vectors, and FP64 scratch for the coarsest level.
 template <class T>
 size_t small_layout(SmallProgram<T>& prog) {
   size_t bytes = 0;
@@ -293,7 +386,8 @@ size_t small_layout(SmallProgram<T>& prog) {
     S.vectors = add(kSmallVectors * n * sizeof(T));
   }
   const SmallLevel<T>& last = prog.level[prog.count - 1];
-  prog.wide = add(2 * static_cast<size_t>(last.view.nx) * last.view.ny * last.view.nz *
+  prog.wide = add((2 * static_cast<size_t>(last.view.nx) * last.view.ny * last.view.nz +
+                   kSmallThreads) *
                   sizeof(double));
   return bytes;
 }

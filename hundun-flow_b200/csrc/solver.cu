@@ -294,18 +294,16 @@ Status Solver::allocate() {
   for (auto& k : k_off) k = add(cells * 8);
   const size_t scalars_off = add(sizeof(Scalars));
   const size_t partials_off = add(sizeof(double) * kBasisChunk * 148 * 8 + 4096);
-  // Dense affine map of the coarsest-level sweeps (one line axis, few cells).
+  // Dense affine map of the coarsest-level line sweeps (few cells).
   const Shape& last = shapes.back();
-  const int last_cells = last.n[0] * last.n[1] * last.n[2];
+  const long long last_cells = static_cast<long long>(last.n[0]) * last.n[1] * last.n[2];
   size_t dense_off = SIZE_MAX;
-  coarse_axis_ = -1;
-  if (last.line_mask != 0 && (last.line_mask & (last.line_mask - 1)) == 0 &&
-      last_cells <= kCoarseDenseMaxCells) {
-    const int axis = last.line_mask == 1 ? 0 : (last.line_mask == 2 ? 1 : 2);
-    if (line_kind(last.n[0], last.n[1], last.n[2], axis) == kLinePcr) {
-      coarse_axis_ = axis;
-      dense_off = add(2 * static_cast<size_t>(last_cells) * last_cells * 8);
-    }
+  if (last.line_mask != 0 && last_cells <= kCoarseDenseMaxCells) {
+    bool pcr = true;
+    for (int a = 0; a < 3; ++a)
+      if (last.line_mask & (1 << a))
+        pcr = pcr && line_kind(last.n[0], last.n[1], last.n[2], a) == kLinePcr;
+    if (pcr) dense_off = add(2 * static_cast<size_t>(last_cells) * last_cells * 8);
   }
   size_t dic_off[2] = {SIZE_MAX, SIZE_MAX};
   if (policy_.preconditioner == HFPS_PRECONDITIONER_IC0) {
@@ -411,7 +409,6 @@ Status Solver::allocate() {
       b.lfac[ax] = reinterpret_cast<float*>(at(o.lf32[ax]));
     }
   }
-  select_small();
   return check(cudaStreamSynchronize(stream_), "allocation");
 }
 
@@ -486,17 +483,24 @@ Status Solver::build_hierarchy() {
     for (int a = 0; a < 3; ++a)
       if (L.lfac[a] != nullptr) launch_line_factors<double>(stream_, L.view(neumann_), a, L.lfac[a]);
   // The coarsest level's sweeps (from any x_in and b) are one affine map;
-  // record its columns once per coefficient update.
+  // record its columns once per coefficient update, axis after axis.
   coarse_dense_ = false;
   if (coarse_op_ != nullptr) {
     const DeviceLevel<double>& D = l64_.back();
-    coarse_dense_ = launch_coarse_line<double, double>(
-        stream_, D.view(neumann_), coarse_op_, nullptr, D.lfac[coarse_axis_],
-        policy_.coarse_sweeps, coarse_axis_, true);
+    int columns = kCoarseColumns;
+    for (int a = 0; a < 3; ++a) {
+      if (!(D.line_mask & (1 << a))) continue;
+      coarse_dense_ = launch_coarse_line<double, double>(stream_, D.view(neumann_), coarse_op_,
+                                                         nullptr, D.lfac[a],
+                                                         policy_.coarse_sweeps, a, columns);
+      if (!coarse_dense_) break;
+      columns = kCoarseColumnsOn;
+    }
   }
   Status st = check(cudaGetLastError(), "hierarchy kernels");
   if (!st) return st;
   select_tail();
+  select_small();
   // Diagonal shortcut (select_diagonal_shortcut, src/solver_mg.cpp:1577-1611).
   diagonal_shortcut_ = false;
   if (policy_.diagonal_shortcut_maximum_ratio != 0.0 &&
@@ -839,17 +843,29 @@ void Solver::coarse_solve(std::vector<DeviceLevel<T>>& levels, bool x_zero) {
   }
 }
 
-// The one-CTA launch covers the point levels from the first of at most
-// kSmallMaxCells cells whose program (shared memory, phases) fits.
+// The one-CTA launch covers the levels from the first of at most
+// kSmallMaxCells cells whose lines fit a warp and whose program (shared
+// memory, phases) fits.  A line hierarchy also needs the dense coarsest map
+// within one CTA's rows, and a level above it: alone it is faster spread over
+// several CTAs (k_coarse_dense).
 void Solver::select_small() {
   small_level_ = -1;
   const int levels = static_cast<int>(l64_.size());
-  if (policy_.null_space != HFPS_NULL_SPACE_NONE || policy_.pre_sweeps > kSmallMaxStages ||
-      policy_.post_sweeps > kSmallMaxStages)
+  if (tail_level_ >= 0 || policy_.null_space != HFPS_NULL_SPACE_NONE ||
+      policy_.pre_sweeps > kSmallMaxStages || policy_.post_sweeps > kSmallMaxStages)
     return;
-  for (int l = 0; l < levels; ++l) {
-    if (l64_[l].line_mask != 0) return;
-    if (l64_[l].cells() > kSmallMaxCells || levels - l > kSmallMaxLevels) continue;
+  const int lines = l64_[0].line_mask;
+  if (lines != 0 && (!coarse_dense_ || l64_.back().cells() > kSmallDenseCells)) return;
+  for (int l = 0; l < levels - (lines != 0 ? 1 : 0); ++l) {
+    const DeviceLevel<double>& L = l64_[l];
+    if (L.cells() > kSmallMaxCells || levels - l > kSmallMaxLevels) continue;
+    const int n[3] = {L.nx, L.ny, L.nz};
+    bool fits = true;
+    for (int a = 0; a < 3; ++a)
+      if (lines & (1 << a))
+        fits = fits && n[a] <= 1 << kSmallMaxSteps &&
+               line_kind(L.nx, L.ny, L.nz, a) == kLinePcr;
+    if (!fits) continue;
     SmallProgram<double> prog;
     if (!small_program(l64_, l, policy_.cycle == 1 ? 2 : 1, true, prog) ||
         small_layout(prog) > kSmallMaxShared)
@@ -871,12 +887,24 @@ bool Solver::small_ops(const std::vector<DeviceLevel<T>>& levels, int first, int
                           static_cast<unsigned>(slot[lv]) << 16;
     return true;
   };
-  if (level == last) return add(kSmallCoarse, l, 0);
+  const int lines = levels[level].line_mask;
+  if (level == last)
+    return lines != 0 ? add(kSmallDense, l, x_zero ? 1 : 0) : add(kSmallCoarse, l, 0);
   const bool chebyshev = levels[level].chebyshev;
   // smooth(): the first step from x = 0 is taken by the start or the gather.
   const auto smoother = [&](int sweeps, bool reverse, bool started) {
     bool ok = true;
-    if (chebyshev) {
+    if (lines != 0) {
+      const int n[3] = {levels[level].nx, levels[level].ny, levels[level].nz};
+      for (int e = 0; e < 3; ++e) {
+        const int a = reverse ? 2 - e : e;
+        if (!(lines & (1 << a))) continue;
+        int steps = 0;
+        while (1 << steps < n[a]) ++steps;
+        for (int p = 0; p < 2 * sweeps; ++p)
+          ok = ok && add(kSmallLine, l, a | ((p + (reverse ? 1 : 0)) & 1) << 2 | steps << 3);
+      }
+    } else if (chebyshev) {
       for (int s = started ? 1 : 0; s < sweeps; ++s) {
         ok = ok && add(kSmallStage, l, s);
         slot[l] ^= 1;
@@ -887,9 +915,9 @@ bool Solver::small_ops(const std::vector<DeviceLevel<T>>& levels, int first, int
     }
     return ok;
   };
-  const int below = level + 1 == last ? kZeroClear
-                                      : (levels[level + 1].chebyshev ? kZeroChebyshev
-                                                                     : kZeroRedBlack);
+  const int below = level + 1 == last || lines != 0
+                        ? kZeroClear
+                        : (levels[level + 1].chebyshev ? kZeroChebyshev : kZeroRedBlack);
   return smoother(policy_.pre_sweeps, false, x_zero) && add(kSmallDefect, l, 0) &&
          add(kSmallGather, l + 1, below) &&
          small_ops(levels, first, level + 1, counter, true, slot, prog) &&
@@ -919,8 +947,10 @@ bool Solver::small_program(const std::vector<DeviceLevel<T>>& levels, int first,
   for (int l = 0; l < count; ++l) {
     prog.level[l].view = levels[first + l].view(neumann_);
     prog.level[l].mask = levels[first + l].coarsen_mask;
+    for (int a = 0; a < 3; ++a) prog.level[l].factors[a] = levels[first + l].lfac[a];
   }
-  if (count > 1)
+  prog.dense = coarse_op_;
+  if (count > 1 && levels[first].line_mask == 0)
     prog.op[prog.ops++] =
         static_cast<unsigned>(kSmallStart) |
         static_cast<unsigned>(levels[first].chebyshev ? kZeroChebyshev : kZeroRedBlack) << 8;

@@ -118,7 +118,7 @@ class Solver {
   // What the producer of `level`'s rhs writes to its x (ZeroKind).
   template <class T>
   ZeroStart<T> zero_start(const std::vector<DeviceLevel<T>>& levels, int level) const;
-  // The smallest point levels as one launch: small_ops appends the phases of
+  // The smallest levels as one launch: small_ops appends the phases of
   // cycle(level, counter), false when they do not fit; small_program builds
   // the program of consecutive visits of the first such level with the given
   // counters, and small_cycle launches it.
@@ -192,15 +192,14 @@ class Solver {
   // The finest level's first pre-smoothing sweep runs on the chunked scan
   // with the zero flags, so the MG entry need not clear x.
   bool first_sweep_zero_{};
-  // Coarsest level in line mode with one line axis and at most
-  // kCoarseDenseMaxCells cells: its coarse_sweeps zebra line sweeps are an
+  // Coarsest level in line mode with at most kCoarseDenseMaxCells cells: its
+  // coarse_sweeps zebra line sweeps along each strong axis are an
   // affine map x_out = P x_in + M b, recorded column by column after every
   // coefficient update and applied as one dense product (P then M, FP64,
   // column-major).
   double* coarse_op_{};
-  int coarse_axis_{-1};
   bool coarse_dense_{};
-  // First level of the one-CTA launch of the smallest point levels (-1: none).
+  // First level of the one-CTA launch of the smallest levels (-1: none).
   int small_level_{-1};
   // First level of the persistent small-level launch (-1: every phase is
   // its own kernel), its PCR width and co-resident grid per precision.
