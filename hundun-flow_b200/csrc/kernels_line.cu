@@ -822,7 +822,9 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
 #undef HFPS_SCAN_LAUNCH
 }
 
-// As many lines per block as its threads have chunks for.
+// As many lines per block as its threads have chunks for, halved (down to one
+// per warp of the load phase) while that leaves fewer than four blocks per SM:
+// with 42 lines of 40 cells per block a level of 1024 lines ran on 25 SMs.
 template <class T>
 void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* fac, int color,
                    long long per_color) {
@@ -833,6 +835,8 @@ void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T*
   sh.rows = (L.nx + sh.chunks - 1) / sh.chunks;
   sh.pitch = sh.rows | 1;
   sh.lines = threads / sh.chunks;
+  while (sh.lines > threads / 32 && per_color < 592LL * sh.lines)
+    sh.lines = std::max(threads / 32, sh.lines / 2);
   const int arrays = 1 + ScanConfig<T>::arrays;
   const size_t smem = static_cast<size_t>(sh.lines) * sh.chunks *
                       (static_cast<size_t>(arrays) * sh.pitch + 4) * sizeof(T);
