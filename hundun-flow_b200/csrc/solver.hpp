@@ -149,6 +149,8 @@ class Solver {
   Status recycle_publish(const double* x, hfps_result& result);
   Status recycle_project(const hfps_control& control, double tol, hfps_result& result);
   Status sync_scalars();
+  // Whether a kernel may read or write the caller's n doubles at p in place.
+  bool in_place(const double* p, size_t n, int memory) const;
   Status copy_in(double* dst, const double* src, size_t n, int memory);
   Status copy_out(double* dst, const double* src, size_t n, int memory);
 
@@ -158,6 +160,7 @@ class Solver {
   std::vector<double> faces_[3];
   std::vector<uint8_t> active_host_;
   bool has_active_{};
+  int device_{};
   bool own_stream_{};
   cudaStream_t stream_{};
   std::string error_;
