@@ -1474,6 +1474,28 @@ __global__ void k_shortcut_ratio(Level<double> L, Reduce red) {
   if (threadIdx.x == 0) red.partials[blockIdx.x] = scratch[0];
 }
 
+// One thread per boundary face of the six sides.
+__global__ void k_neumann_faces(Level<double> L, Scalars* scalars) {
+  grid_dependency_sync();
+  const int nx = L.nx, ny = L.ny, nz = L.nz;
+  const int sides[3] = {ny * nz, nx * nz, nx * ny};
+  const int total = 2 * (sides[0] + sides[1] + sides[2]);
+  int bad = 0;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    int r = t, axis = 0;
+    while (r >= 2 * sides[axis]) r -= 2 * sides[axis++];
+    const int high = r >= sides[axis] ? 1 : 0;
+    if (!((L.neumann >> (2 * axis + high)) & 1u)) continue;
+    r -= high * sides[axis];
+    double f;
+    if (axis == 0) f = L.fx[(high ? nx : 0) + (nx + 1) * r];
+    else if (axis == 1) f = L.fy[r % nx + nx * ((high ? ny : 0) + (ny + 1) * (r / nx))];
+    else f = L.fz[r + (high ? nx * ny * nz : 0)];
+    bad |= f != 0.0;
+  }
+  if (bad) atomicOr(&scalars->marks, 2u);
+}
+
 template <class TO, class TI>
 __global__ void k_convert(size_t n, const TI* __restrict__ src,
                           TO* __restrict__ dst) {
@@ -1891,6 +1913,12 @@ void launch_correct_flux(cudaStream_t s, int nx, int ny, int nz, unsigned neuman
 void launch_shortcut_ratio(cudaStream_t s, const Level<double>& L,
                            Reduce red) {
   launch(k_shortcut_ratio, reduction_blocks(HFPS_CELLS(L)), kThreads, 0, s, L, red);
+}
+void launch_neumann_faces(cudaStream_t s, const Level<double>& L, Scalars* scalars) {
+  const long long faces = 2 * (static_cast<long long>(L.ny) * L.nz +
+                               static_cast<long long>(L.nx) * L.nz +
+                               static_cast<long long>(L.nx) * L.ny);
+  launch(k_neumann_faces, grid_for(faces), kThreads, 0, s, L, scalars);
 }
 template <class TO, class TI>
 void launch_convert(cudaStream_t s, size_t n, const TI* src, TO* dst) {

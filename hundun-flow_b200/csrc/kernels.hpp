@@ -141,11 +141,12 @@ void launch_line_factors(cudaStream_t s, const Level<T>& L, int axis, T* fac);
 // One zebra colour of line relaxation along `axis`, x and b in layout hx
 // (split rows only with the scan solve, axis 1 or 2).  zero_other: the other
 // colour's x is known to be zero (not read); zero_self: this colour's x is
-// (the first pass and the first sweep of a cycle started from x = 0).
+// (the first pass and the first sweep of a cycle started from x = 0).  ends: a
+// Neumann boundary face of the level may be nonzero (launch_neumann_faces).
 template <class T>
 void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
                       const T* fac, T* scratch, int axis, int color, int hx = 0,
-                      bool zero_other = false, bool zero_self = false);
+                      bool zero_other = false, bool zero_self = false, bool ends = true);
 // Coarsest level in line mode with x/rhs resident in shared memory; returns
 // false when the level is too large for that form.  With kCoarseColumns,
 // launches 2n blocks that write the columns of the sweeps' affine map x_out =
@@ -417,6 +418,8 @@ void launch_beta_coefficients(cudaStream_t s, int nx, int ny, int nz,
                               double* fz);
 void launch_shortcut_ratio(cudaStream_t s, const Level<double>& L,
                            Reduce red);
+// Sets bit 1 of scalars->marks when any Neumann boundary face is not zero.
+void launch_neumann_faces(cudaStream_t s, const Level<double>& L, Scalars* scalars);
 template <class TO, class TI>
 void launch_convert(cudaStream_t s, size_t n, const TI* src, TO* dst);
 

@@ -50,7 +50,6 @@ struct LineRhs {
   int fbase[2], fstride[2], fhigh[2];
   int off[4];
   bool keep[4];
-  bool self[4];   // the neighbour is the cell itself (outside the level)
   T end_low, end_high;   // line-end boundary faces (rows 0 and extent-1)
   bool lkeep_low, lkeep_high;
 
@@ -79,7 +78,9 @@ struct LineRhs {
     (void)nz;
   }
 
-  __device__ LineRhs(const Level<T>& L, int fa, int fb, int hx) {
+  // own_zero: this colour's x counts as zero, so a neighbour that is the cell
+  // itself is left out.
+  __device__ LineRhs(const Level<T>& L, int fa, int fb, int hx, bool own_zero = false) {
     int i0, j0, k0;
     line_cell(AXIS, fa, fb, 0, i0, j0, k0);
     const int idx[3] = {i0, j0, k0};
@@ -99,10 +100,8 @@ struct LineRhs {
       }
       off[2 * n] = low_in ? lo : 0;
       off[2 * n + 1] = high_in ? hi : 0;
-      self[2 * n] = !low_in;
-      self[2 * n + 1] = !high_in;
-      keep[2 * n] = low_in || ((L.neumann >> (2 * a)) & 1u);
-      keep[2 * n + 1] = high_in || ((L.neumann >> (2 * a + 1)) & 1u);
+      keep[2 * n] = low_in || (!own_zero && ((L.neumann >> (2 * a)) & 1u));
+      keep[2 * n + 1] = high_in || (!own_zero && ((L.neumann >> (2 * a + 1)) & 1u));
     }
     const T* lface;
     int lbase, lstride, lhigh;
@@ -113,29 +112,25 @@ struct LineRhs {
     lkeep_high = (L.neumann >> (2 * AXIS + 1)) & 1u;
   }
 
-  // Row s, c its vector index.  MODE kScanFresh: x is zero everywhere and
-  // not read.  kScanOwnZero: this colour's x is zero; its values (the cell
-  // itself, read where a neighbour lies outside the level) are still loaded,
-  // so that every load stays unconditional, and then replaced by zero.
-  template <int MODE>
+  // Row s, c its vector index.  MODE kScanFresh: x is zero everywhere, so the
+  // row is the rhs alone (every term is a finite face times zero).
+  // ENDS: a Neumann
+  // face at a line end may be nonzero; otherwise the end terms are exact zeros
+  // and the cell's own x is not read.
+  template <int MODE, bool ENDS>
   __device__ __forceinline__ T row(const T* x, const T* __restrict__ rhs, int c,
                                    int s, int extent) const {
     T d = __ldg(rhs + c);
+    if (MODE == kScanFresh) return d;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int f = fbase[n] + s * fstride[n];
-      T lo = T(0), hi = T(0);
-      if (MODE != kScanFresh) {
-        lo = __ldg(x + c + off[2 * n]);
-        hi = __ldg(x + c + off[2 * n + 1]);
-      }
-      if (MODE == kScanOwnZero) {
-        lo = self[2 * n] ? T(0) : lo;
-        hi = self[2 * n + 1] ? T(0) : hi;
-      }
+      const T lo = __ldg(x + c + off[2 * n]);
+      const T hi = __ldg(x + c + off[2 * n + 1]);
       d += __ldg(face[n] + f) * (keep[2 * n] ? lo : T(0));
       d += __ldg(face[n] + f + fhigh[n]) * (keep[2 * n + 1] ? hi : T(0));
     }
+    if (!ENDS) return d;
     const T self_value = MODE == kScanNormal ? x[c] : T(0);
     const T dl = d + end_low * (lkeep_low ? self_value : T(0));
     d = s == 0 ? dl : d;
@@ -277,19 +272,21 @@ __global__ void k_scan_factors(Level<T> L, int axis, T* __restrict__ fac) {
 // One zebra colour: blockDim = (LPB lines, S chunks), chunk q holds rows
 // [q*m, min(extent, (q+1)*m) - 1] with m <= ScanConfig<T>::rows.  Shared memory holds
 // the chunk compositions: forward (A, B) and backward (A, B), S x LPB each.
-template <class T, int AXIS, int LPB, int MODE, bool SPLIT>
+template <class T, int AXIS, int LPB, int MODE, bool SPLIT, bool ENDS>
 __global__ void __launch_bounds__(ScanConfig<T>::threads)
     k_line_scan_color(Level<T> L, T* x, const T* __restrict__ rhs,
-                      const T* __restrict__ fac, int color, int m, int hx) {
+                      const T* __restrict__ fac, int color, int m, int hx, bool own_zero) {
   grid_dependency_sync();
   extern __shared__ unsigned char scan_smem[];
   const int S = blockDim.y;
+  constexpr bool kSym = ScanConfig<T>::symmetric;
+  constexpr int kScanRows = ScanConfig<T>::rows;
   T* fA = reinterpret_cast<T*>(scan_smem);
   T* fB = fA + S * LPB;
   T* bA = fB + S * LPB;
   T* bB = bA + S * LPB;
   const int extent = line_extent(AXIS, L.nx, L.ny, L.nz);
-  const int a_extent = AXIS == 0 ? L.ny : L.nx;
+  const int a_extent = L.nx;
   const int b_extent = AXIS == 2 ? L.ny : L.nz;
   const int ha = (a_extent + 1) >> 1;
   const ScanLayout lay{extent, ha * b_extent, false};
@@ -314,7 +311,6 @@ __global__ void __launch_bounds__(ScanConfig<T>::threads)
   const int rows = valid ? max(0, min(m, extent - r0)) : 0;
   const int row = lay.colour_lines;
   const int tt = valid ? t : 0;
-  constexpr bool kSym = ScanConfig<T>::symmetric;
   const T* inv = fac + lay.cell(0, color, 0, tt);
   const T* lf = fac + lay.cell(1, color, 0, tt);
   const T* uf = fac + lay.cell(kSym ? 1 : 2, color, 0, tt);
@@ -335,12 +331,12 @@ __global__ void __launch_bounds__(ScanConfig<T>::threads)
 
   // Pass 1: right-hand sides (scaled by 1/den unless symmetric), and the
   // forward composition.
-  const LineRhs<T, AXIS, SPLIT> lr(L, valid ? fa : 0, valid ? fb : 0, hx);
-  constexpr int kScanRows = ScanConfig<T>::rows;
+  const LineRhs<T, AXIS, SPLIT> lr(L, valid ? fa : 0, valid ? fb : 0, hx,
+                                    MODE == kScanOwnZero || (!ENDS && own_zero));
   T v[kScanRows];
 #pragma unroll
   for (int u = 0; u < kScanRows; ++u) {
-    v[u] = lr.template row<MODE>(x, rhs, base + srow(u) * stride, srow(u), extent);
+    v[u] = lr.template row<MODE, ENDS>(x, rhs, base + srow(u) * stride, srow(u), extent);
     if constexpr (!kSym) v[u] = v[u] * __ldg(inv + srow(u) * row);
   }
   T A = T(1), B = T(0);
@@ -792,9 +788,16 @@ ScanShape scan_shape(long long per_color, int extent) {
   return sh;
 }
 
+// Without end terms the FP64 kernel needs 128 registers instead of 165, so four
+// blocks share an SM: a level-0 pass of the split 256^3 level went from 144 to
+// 122 us and one of level 1 from 43 to 35.  In natural order the fourth block's
+// half-used sectors cost more than it gives (456x256x52 y-lines 65.6 -> 71 us),
+// and levels that three blocks per SM hold anyway gain nothing (64x256x64 9.9 ->
+// 11.0 us, 32x256x32 7.3 -> 8.3): those keep the kernel with the end terms,
+// which are exact zeros then.
 struct ScanFlags {
   int hx;
-  bool zero_other, zero_self;
+  bool zero_other, zero_self, ends;
 };
 
 template <class T, int AXIS, int LPB>
@@ -803,23 +806,34 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
   const int blocks = static_cast<int>((per_color + LPB - 1) / LPB);
   const size_t smem = static_cast<size_t>(4) * sh.chunks * LPB * sizeof(T);
   const dim3 block(LPB, sh.chunks);
+  // Without end terms the zero flag is an argument of the ordinary kernel (a
+  // kernel of its own takes more registers); with them it is a mode.
+  const bool ends = f.ends || f.hx == 0 || blocks <= 3 * 148;
   const int mode = f.zero_other && f.zero_self ? kScanFresh
-                                               : (f.zero_self ? kScanOwnZero : kScanNormal);
+                                               : (f.zero_self && ends ? kScanOwnZero : kScanNormal);
   const bool split = f.hx != 0;
+#define HFPS_SCAN_RUN(MODE, SPLIT, ENDS)                                                    \
+  launch(k_line_scan_color<T, AXIS, LPB, MODE, SPLIT, ENDS>, blocks, block, smem, s, L, x, b, \
+         fac, color, sh.rows, f.hx, f.zero_self)
+#define HFPS_SCAN_ENDS(MODE, SPLIT) HFPS_SCAN_RUN(MODE, SPLIT, true)
 #define HFPS_SCAN_LAUNCH(MODE, SPLIT)                                                       \
-  launch(k_line_scan_color<T, AXIS, LPB, MODE, SPLIT>, blocks, block, smem, s, L, x, b, fac, \
-         color, sh.rows, f.hx)
+  do {                                                                                      \
+    if (ends) HFPS_SCAN_RUN(MODE, SPLIT, true);                                             \
+    else HFPS_SCAN_RUN(MODE, SPLIT, false);                                                 \
+  } while (0)
   if (mode == kScanFresh) {
     if (split) HFPS_SCAN_LAUNCH(kScanFresh, true);
     else HFPS_SCAN_LAUNCH(kScanFresh, false);
   } else if (mode == kScanOwnZero) {
-    if (split) HFPS_SCAN_LAUNCH(kScanOwnZero, true);
-    else HFPS_SCAN_LAUNCH(kScanOwnZero, false);
+    if (split) HFPS_SCAN_ENDS(kScanOwnZero, true);
+    else HFPS_SCAN_ENDS(kScanOwnZero, false);
   } else {
     if (split) HFPS_SCAN_LAUNCH(kScanNormal, true);
     else HFPS_SCAN_LAUNCH(kScanNormal, false);
   }
 #undef HFPS_SCAN_LAUNCH
+#undef HFPS_SCAN_ENDS
+#undef HFPS_SCAN_RUN
 }
 
 // As many lines per block as its threads have chunks for, halved (down to one
@@ -909,7 +923,7 @@ void launch_line_factors(cudaStream_t s, const Level<T>& L, int axis, T* fac) {
 template <class T>
 void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
                       const T* fac, T* scratch, int axis, int color, int hx,
-                      bool zero_other, bool zero_self) {
+                      bool zero_other, bool zero_self, bool ends) {
   (void)scratch;
   const int extent = line_extent(axis, L.nx, L.ny, L.nz);
   const int a_extent = axis == 0 ? L.ny : L.nx;
@@ -923,7 +937,7 @@ void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
       return;
     }
     const ScanShape sh = scan_shape<T>(per_color, extent);
-    const ScanFlags f{hx, zero_other, zero_self};
+    const ScanFlags f{hx, zero_other, zero_self, ends};
     if (axis == 1) launch_scan_axis<T, 1>(s, L, x, b, fac, color, per_color, sh, f);
     else launch_scan_axis<T, 2>(s, L, x, b, fac, color, per_color, sh, f);
     return;
@@ -988,9 +1002,9 @@ template void launch_line_factors<double>(cudaStream_t, const Level<double>&, in
 template void launch_line_factors<float>(cudaStream_t, const Level<float>&, int, float*);
 template void launch_line_pass<double>(cudaStream_t, const Level<double>&, double*,
                                        const double*, const double*, double*, int, int, int,
-                                       bool, bool);
+                                       bool, bool, bool);
 template void launch_line_pass<float>(cudaStream_t, const Level<float>&, float*, const float*,
-                                      const float*, float*, int, int, int, bool, bool);
+                                      const float*, float*, int, int, int, bool, bool, bool);
 template bool launch_coarse_line<double, double>(cudaStream_t, const Level<double>&, double*,
                                                  const double*, const double*, int, int, int);
 template bool launch_coarse_line<float, double>(cudaStream_t, const Level<double>&, float*,

@@ -163,8 +163,8 @@ Status Solver::create(const hfps_geometry& g, const hfps_policy& policy,
   s->ny_ = g.ny;
   s->nz_ = g.nz;
   s->neumann_ = neumann;
-  cudaGetDevice(&s->device_);
   s->policy_ = policy;
+  cudaGetDevice(&s->device_);
   const double* src[3] = {g.x_faces, g.y_faces, g.z_faces};
   const int n[3] = {g.nx, g.ny, g.nz};
   for (int a = 0; a < 3; ++a) {
@@ -437,7 +437,6 @@ Status Solver::copy_out(double* dst, const double* src, size_t n, int memory) {
                "copy out");
 }
 
-// One channel of aggregate_tensor_channel over the axes the fine level
 // The caller's array is used in place when it is device memory of the solver's
 // GPU at a double's alignment, inside one allocation; anything else goes
 // through the staging vectors, where cudaMemcpyAsync takes any address it can
@@ -469,6 +468,7 @@ bool Solver::in_place(const double* p, size_t n, int memory) const {
          n * sizeof(double) <= bytes - (at - base);
 }
 
+// One channel of aggregate_tensor_channel over the axes the fine level
 // coarsens, in x->y->z order (src/solver_mg.cpp:1706-1856).
 void Solver::aggregate_channel(int level, int face_axis, const double* src,
                                double* dst) {
@@ -533,6 +533,18 @@ Status Solver::build_hierarchy() {
   if (!st) return st;
   select_tail();
   select_small();
+  line_ends_ = true;
+  if (l64_[0].line_mask != 0) {
+    st = check(cudaMemsetAsync(&d_scalars_->marks, 0, sizeof(unsigned), stream_), "boundary faces");
+    if (!st) return st;
+    launch_neumann_faces(stream_, l64_[0].view(neumann_), d_scalars_);
+    st = check(cudaMemcpyAsync(&h_scalars_->marks, &d_scalars_->marks, sizeof(unsigned),
+                               cudaMemcpyDeviceToHost, stream_),
+               "boundary faces");
+    if (st) st = check(cudaStreamSynchronize(stream_), "boundary faces");
+    if (!st) return st;
+    line_ends_ = (h_scalars_->marks & 2u) != 0;
+  }
   // Diagonal shortcut (select_diagonal_shortcut, src/solver_mg.cpp:1577-1611).
   diagonal_shortcut_ = false;
   if (policy_.diagonal_shortcut_maximum_ratio != 0.0 &&
@@ -836,7 +848,8 @@ void Solver::smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
       for (int pass = 0; pass < 2; ++pass) {
         const bool fresh = x_zero && one_axis && s == 0;
         launch_line_pass<T>(stream_, view, L.x, L.b, L.lfac[axis], L.r, axis,
-                            (first + pass) & 1, L.split, fresh && pass == 0, fresh);
+                            (first + pass) & 1, L.split, fresh && pass == 0, fresh,
+                            line_ends_);
       }
   };
   if (reverse) {
@@ -2393,7 +2406,8 @@ Status Solver::profile_kernel(int kernel, int repetitions, double* ms,
     if (L.line_mask != 0) {
       int axis = 0;
       while (!(L.line_mask & (1 << axis))) ++axis;
-      launch_line_pass<T>(stream_, view, L.x, L.b, L.lfac[axis], L.r, axis, 0, L.split);
+      launch_line_pass<T>(stream_, view, L.x, L.b, L.lfac[axis], L.r, axis, 0, L.split, false,
+                          false, line_ends_);
       return 28.0 / 8.0 * sizeof(T);
     }
     if (L.chebyshev) {

@@ -155,12 +155,12 @@ class Solver {
   Status copy_out(double* dst, const double* src, size_t n, int memory);
 
   int nx_{}, ny_{}, nz_{};
+  int device_{};
   unsigned neumann_{};
   hfps_policy policy_{};
   std::vector<double> faces_[3];
   std::vector<uint8_t> active_host_;
   bool has_active_{};
-  int device_{};
   bool own_stream_{};
   cudaStream_t stream_{};
   std::string error_;
@@ -192,6 +192,10 @@ class Solver {
   bool coefficients_ready_{};
   bool mixed_ready_{};
   bool diagonal_shortcut_{};
+  // Some Neumann boundary face is nonzero (set_beta and assemble make them
+  // zero), so line passes must add the end terms.  Coarse boundary faces are
+  // sums of the finest ones.
+  bool line_ends_{true};
   // The finest level's first pre-smoothing sweep runs on the chunked scan
   // with the zero flags, so the MG entry need not clear x.
   bool first_sweep_zero_{};
