@@ -723,14 +723,9 @@ __global__ void __launch_bounds__(kTileX * kTileY)
 }
 
 // ---------------------------------------------------------------------------
-// Cold-path diagonal IC(0) (ColdPressureIccg, src/solver_iccg.hpp:224-293;
-// ColdPressureDilu, src/solver_cold.hpp:484-560, identical on the symmetric
-// pressure rows).  The factorisation and both triangular sweeps follow the
-// reference's lexicographic order exactly: a cell depends only on its lower
-// (resp. upper) neighbours, which all lie on the previous wavefront plane
-// i + j + k = t - 1 (resp. t + 1), so every plane is one parallel launch and
-// each cell's arithmetic is the reference's, operation for operation.  The
-// couplings are the IBM-masked level-0 face coefficients.
+// Cold-path diagonal IC(0): the row diagonals it starts from (factorisation
+// and sweeps in kernels_dic.cu).  The couplings are the IBM-masked level-0
+// face coefficients.
 
 // Row diagonal of the decorated operator: identity on solid cells; a link to
 // a solid cell or a Neumann boundary face leaves the row and its coefficient
@@ -768,69 +763,6 @@ __global__ void k_dic_rows(int nx, int ny, int nz, unsigned neumann, const doubl
     }
     out[c] = d;
   }
-}
-
-// Cell (i, j, k) of wavefront plane t handled by this thread, or false.
-__device__ __forceinline__ bool plane_cell(int t, int nx, int ny, int nz, int& i, int& j,
-                                           int& k) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ny * nz) return false;
-  k = q / ny;
-  j = q - k * ny;
-  i = t - j - k;
-  return i >= 0 && i < nx;
-}
-
-__global__ void k_dic_pivots(int t, Level<double> L, const double* rows, double* inv,
-                             Scalars* scalars) {
-  grid_dependency_sync();
-  int i, j, k;
-  if (!plane_cell(t, L.nx, L.ny, L.nz, i, j, k)) return;
-  const int c = i + L.nx * (j + L.ny * k);
-  const int plane = L.nx * L.ny;
-  double pivot = rows[c];
-  // lower couplings: the cell's own x-, y-, z- faces
-  if (i > 0) {
-    const double lower = L.fx[face_x_index(L, c, j, k)];
-    pivot -= lower * lower * inv[c - 1];
-  }
-  if (j > 0) {
-    const double lower = L.fy[face_y_index(L, c, k)];
-    pivot -= lower * lower * inv[c - L.nx];
-  }
-  if (k > 0) {
-    const double lower = L.fz[c];
-    pivot -= lower * lower * inv[c - plane];
-  }
-  if (!(pivot > 0) || !isfinite(pivot)) atomicOr(&scalars->flags, 1);
-  inv[c] = 1 / pivot;
-}
-
-__global__ void k_dic_forward(int t, Level<double> L, const double* in, double* out,
-                              const double* inv) {
-  grid_dependency_sync();
-  int i, j, k;
-  if (!plane_cell(t, L.nx, L.ny, L.nz, i, j, k)) return;
-  const int c = i + L.nx * (j + L.ny * k);
-  double value = in[c];
-  if (i > 0) value += L.fx[face_x_index(L, c, j, k)] * out[c - 1];
-  if (j > 0) value += L.fy[face_y_index(L, c, k)] * out[c - L.nx];
-  if (k > 0) value += L.fz[c] * out[c - L.nx * L.ny];
-  out[c] = value * inv[c];
-}
-
-__global__ void k_dic_backward(int t, Level<double> L, double* out, const double* inv) {
-  grid_dependency_sync();
-  int i, j, k;
-  if (!plane_cell(t, L.nx, L.ny, L.nz, i, j, k)) return;
-  const int c = i + L.nx * (j + L.ny * k);
-  const int plane = L.nx * L.ny;
-  double value = 0;
-  // upper couplings: the lower face of the next cell along each axis
-  if (i + 1 < L.nx) value += L.fx[face_x_index(L, c, j, k) + 1] * out[c + 1];
-  if (j + 1 < L.ny) value += L.fy[face_y_index(L, c, k) + L.nx] * out[c + L.nx];
-  if (k + 1 < L.nz) value += L.fz[c + plane] * out[c + plane];
-  out[c] += value * inv[c];
 }
 
 // ---------------------------------------------------------------------------
@@ -1766,22 +1698,6 @@ void launch_dic_rows(cudaStream_t s, int nx, int ny, int nz, unsigned neumann,
                      const uint8_t* active, double* out) {
   launch(k_dic_rows, grid_for(static_cast<long long>(nx) * ny * nz), kThreads, 0, s, nx, ny, nz,
          neumann, diag, fx, fy, fz, active, out);
-}
-int dic_planes(const Level<double>& L) { return L.nx + L.ny + L.nz - 2; }
-static int plane_blocks(const Level<double>& L) {
-  return static_cast<int>((static_cast<long long>(L.ny) * L.nz + kThreads - 1) / kThreads);
-}
-void launch_dic_pivots(cudaStream_t s, const Level<double>& L, const double* rows, double* inv,
-                       Scalars* scalars) {
-  for (int t = 0; t < dic_planes(L); ++t)
-    launch(k_dic_pivots, plane_blocks(L), kThreads, 0, s, t, L, rows, inv, scalars);
-}
-void launch_dic_apply(cudaStream_t s, const Level<double>& L, const double* in, double* out,
-                      const double* inv) {
-  for (int t = 0; t < dic_planes(L); ++t)
-    launch(k_dic_forward, plane_blocks(L), kThreads, 0, s, t, L, in, out, inv);
-  for (int t = dic_planes(L) - 1; t >= 0; --t)
-    launch(k_dic_backward, plane_blocks(L), kThreads, 0, s, t, L, out, inv);
 }
 void launch_bicg_direction(cudaStream_t s, int n, double* p, const double* r, const double* v,
                            double beta, double omega) {

@@ -352,14 +352,16 @@ void launch_correct_flux(cudaStream_t s, int nx, int ny, int nz, unsigned neuman
 void launch_dic_rows(cudaStream_t s, int nx, int ny, int nz, unsigned neumann,
                      const double* diag, const double* fx, const double* fy, const double* fz,
                      const uint8_t* active, double* out);
-// Wavefront planes i + j + k = t of a level: nx + ny + nz - 2.
-int dic_planes(const Level<double>& L);
-// Inverse pivots, plane by plane (flags bit 0 on a non-positive pivot).
+// Doubles of the sweeps' tickets and tile borders (kernels_dic.cu).
+size_t dic_border_values(int nx, int ny, int nz);
+// Inverse pivots (flags bit 0 on a non-positive pivot; bit 4 when a wait
+// between blocks ran out).
 void launch_dic_pivots(cudaStream_t s, const Level<double>& L, const double* rows, double* inv,
-                       Scalars* scalars);
-// out = M^{-1} in: forward then backward sweep, plane by plane.
+                       double* border, Scalars* scalars);
+// out = M^{-1} in: forward then backward sweep (flags bit 4 as above); out must
+// not alias in.
 void launch_dic_apply(cudaStream_t s, const Level<double>& L, const double* in, double* out,
-                      const double* inv);
+                      const double* inv, double* border, Scalars* scalars);
 void launch_bicg_direction(cudaStream_t s, int n, double* p, const double* r, const double* v,
                            double beta, double omega);
 // s = r - alpha v, with |s|^2 through red.

@@ -125,7 +125,6 @@ Status Solver::check(cudaError_t e, const char* what) {
 Solver::~Solver() {
   if (stream_ != nullptr) cudaStreamSynchronize(stream_);
   clear_mg_graphs();
-  if (dic_graph_ != nullptr) cudaGraphExecDestroy(dic_graph_);
   if (h_scalars_ != nullptr) cudaFreeHost(h_scalars_);
   if (scalars_ready_ != nullptr) cudaEventDestroy(scalars_ready_);
   if (arena_ != nullptr) cudaFree(arena_);
@@ -306,10 +305,11 @@ Status Solver::allocate() {
         pcr = pcr && line_kind(last.n[0], last.n[1], last.n[2], a) == kLinePcr;
     if (pcr) dense_off = add(2 * static_cast<size_t>(last_cells) * last_cells * 8);
   }
-  size_t dic_off[2] = {SIZE_MAX, SIZE_MAX};
+  size_t dic_off[3] = {SIZE_MAX, SIZE_MAX, SIZE_MAX};
   if (policy_.preconditioner == HFPS_PRECONDITIONER_IC0) {
     dic_off[0] = add(cells * 8);
     dic_off[1] = add(cells * 8);
+    dic_off[2] = add(dic_border_values(nx_, ny_, nz_) * sizeof(double));
   }
   arena_bytes_ = bytes;
   Status st = check(cudaMalloc(&arena_, arena_bytes_), "device arena");
@@ -365,6 +365,7 @@ Status Solver::allocate() {
   if (dic_off[0] != SIZE_MAX) {
     dic_rows_ = reinterpret_cast<double*>(at(dic_off[0]));
     dic_inv_ = reinterpret_cast<double*>(at(dic_off[1]));
+    dic_border_ = reinterpret_cast<double*>(at(dic_off[2]));
   }
   l64_.resize(levels);
   l32_.resize(levels);
@@ -590,7 +591,7 @@ Status Solver::build_hierarchy() {
 
 // Cold-path IC(0) factorisation from the coefficients still staged in
 // user_ (diagonal, unmasked faces): decorated row diagonals, then the
-// inverse pivots plane by plane (ColdPressureIccg::prepare,
+// inverse pivots (ColdPressureIccg::prepare,
 // src/solver_iccg.hpp:236-256).
 Status Solver::dic_factor() {
   if (dic_rows_ == nullptr) return {};
@@ -599,7 +600,7 @@ Status Solver::dic_factor() {
   if (!st) return st;
   launch_dic_rows(stream_, nx_, ny_, nz_, neumann_, user_[0], user_[1], user_[2], user_[3],
                   d_active_, dic_rows_);
-  launch_dic_pivots(stream_, L0, dic_rows_, dic_inv_, d_scalars_);
+  launch_dic_pivots(stream_, L0, dic_rows_, dic_inv_, dic_border_, d_scalars_);
   st = sync_scalars();
   if (!st) return st;
   if (h_scalars_->flags & 1) {
@@ -1273,32 +1274,14 @@ Status Solver::mg_apply(bool mixed, const double* r, double* z) {
   return check(cudaGraphLaunch(exec, stream_), "graph launch");
 }
 
-Status Solver::dic_apply() {
-  const Level<double> L0 = l64_[0].view(neumann_);
-  if (!use_graphs_) {
-    launch_dic_apply(stream_, L0, kr_, kz_, dic_inv_);
-    launches_ += 2 * static_cast<uint64_t>(dic_planes(L0));
-    return check(cudaGetLastError(), "IC(0) launch");
-  }
-  if (dic_graph_ == nullptr) {
-    cudaGraph_t graph = nullptr;
-    Status st = check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal),
-                      "graph capture begin");
-    if (!st) return st;
-    launch_dic_apply(stream_, L0, kr_, kz_, dic_inv_);
-    st = check(cudaStreamEndCapture(stream_, &graph), "graph capture end");
-    if (!st) return st;
-    cudaGraphGetNodes(graph, nullptr, &dic_nodes_);
-    st = check(cudaGraphInstantiate(&dic_graph_, graph, 0), "graph instantiate");
-    cudaGraphDestroy(graph);
-    if (!st) return st;
-  }
-  launches_ += dic_nodes_;
-  return check(cudaGraphLaunch(dic_graph_, stream_), "graph launch");
+Status Solver::dic_apply(const double* r, double* z) {
+  launch_dic_apply(stream_, l64_[0].view(neumann_), r, z, dic_inv_, dic_border_, d_scalars_);
+  launches_ += 2;
+  return check(cudaGetLastError(), "IC(0) launch");
 }
 
 Status Solver::precondition(bool mixed) {
-  if (policy_.preconditioner == HFPS_PRECONDITIONER_IC0) return dic_apply();
+  if (policy_.preconditioner == HFPS_PRECONDITIONER_IC0) return dic_apply(kr_, kz_);
   return mg_apply(mixed);
 }
 
@@ -1309,9 +1292,17 @@ Status Solver::sync_scalars() {
   if (!st) return st;
   st = check(cudaStreamSynchronize(stream_), "solver step");
   if (!st) return st;
+  return wait_status();
+}
+
+// Waits between blocks that ran out (the scalars are on the host).
+Status Solver::wait_status() {
   if (h_scalars_->flags & 8)
     return fail(HFPS_NUMERICAL_FAILURE, kDetailNumeric,
                 "small-level kernel: a grid barrier timed out");
+  if (h_scalars_->flags & 16)
+    return fail(HFPS_NUMERICAL_FAILURE, kDetailNumeric,
+                "IC(0) sweep: a wait between blocks timed out");
   return {};
 }
 
@@ -1432,9 +1423,8 @@ Status Solver::krylov_pcg(const hfps_control& control, hfps_result& result,
     }
     st = check(cudaEventSynchronize(scalars_ready_), "solver step");
     if (!st) return st;
-    if (h_scalars_->flags & 8)
-      return fail(HFPS_NUMERICAL_FAILURE, kDetailNumeric,
-                  "small-level kernel: a grid barrier timed out");
+    st = wait_status();
+    if (!st) return st;
     result.iterations = it;
     // A breakdown flag comes from p.Ap of this iteration (the reference
     // stops before counting it) or from the r.z that formed this direction

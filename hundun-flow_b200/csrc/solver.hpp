@@ -101,7 +101,7 @@ class Solver {
   void clear_mg_graphs();
   // z = M r on kr_/kz_ with the policy's preconditioner (MG or cold IC(0)).
   Status precondition(bool mixed);
-  Status dic_apply();
+  Status dic_apply(const double* r, double* z);
   Status dic_factor();
   Status krylov_bicgstab(const hfps_control& control, hfps_result& result,
                          double* history, uint32_t capacity);
@@ -149,6 +149,7 @@ class Solver {
   Status recycle_publish(const double* x, hfps_result& result);
   Status recycle_project(const hfps_control& control, double tol, hfps_result& result);
   Status sync_scalars();
+  Status wait_status();
   // Whether a kernel may read or write the caller's n doubles at p in place.
   bool in_place(const double* p, size_t n, int memory) const;
   Status copy_in(double* dst, const double* src, size_t n, int memory);
@@ -236,12 +237,10 @@ class Solver {
   double* rc_image_[kRecycleMax]{};   // projection scratch: A d_i
   bool rc_capture_{}, rc_guard_only_{}, rc_cycle_active_{}, rc_pending_{};
   int rc_count_{}, rc_oldest_{};
-  // Cold-path IC(0): decorated row diagonals and inverse pivots (level 0),
-  // and the captured wavefront apply (kr_ -> kz_).
+  // Cold-path IC(0): decorated row diagonals and inverse pivots (level 0).
   double* dic_rows_{};
   double* dic_inv_{};
-  cudaGraphExec_t dic_graph_{};
-  size_t dic_nodes_{};
+  double* dic_border_{};      // its sweeps' tickets and tile borders
   // The MG application captured as one CUDA graph per (precision slot,
   // input, output) buffers: the PCG uses kr_/kz_, FGMRES every basis
   // column's V_j/Z_j directly (no copies into fixed buffers).
