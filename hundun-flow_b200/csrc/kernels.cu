@@ -384,7 +384,9 @@ __global__ void __launch_bounds__(kRowThreads)
 // clamps at a level edge the clamped load holds the same cell.  Each fine
 // value is then formed exactly as prolongate_cell forms it (same weights,
 // terms and order), so results are bit-identical to k_prolongate<T, 5>.
-template <class T, class CPos>
+// EVEN: only the cells with i + k even, the zebra colour that the line pass
+// that follows reads; it overwrites the other one without reading it.
+template <class T, class CPos, bool EVEN>
 __global__ void __launch_bounds__(kRowThreads)
     k_prolongate_xz(Level<T> F, T* __restrict__ x, Level<T> C, const T* __restrict__ cx,
                     int hx, CPos cpos) {
@@ -414,7 +416,7 @@ __global__ void __launch_bounds__(kRowThreads)
 #pragma unroll
     for (int dx = 0; dx < 2; ++dx) {
       const int i = 2 * p + dx, k = 2 * q + dz;
-      const bool in = i < F.nx && k < F.nz;
+      const bool in = i < F.nx && k < F.nz && !(EVEN && dx != dz);
       fluid[dz][dx] = in && F.fluid[i + F.nx * (j + F.ny * k)] != 0;
       old[dz][dx] = in ? x[2 * hx * (j + F.ny * k) + dx * hx + p] : T(0);
     }
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(kRowThreads)
     for (int dx = 0; dx < 2; ++dx) {
       const int i = 2 * p + dx;
       if (i >= F.nx) break;
+      if (EVEN && dx != dz) continue;
       int xl, xr;
       double xw;
       interp_axis(i, 1, C.nx, xl, xr, xw);
@@ -1555,15 +1558,18 @@ void launch_defect_restrict(cudaStream_t s, const Level<T>& F, const T* x,
 }
 template <class T>
 void launch_prolongate(cudaStream_t s, const Level<T>& F, T* x,
-                       const Level<T>& C, const T* cx, int mask, int hx, int hxc) {
+                       const Level<T>& C, const T* cx, int mask, int hx, int hxc,
+                       bool even_only) {
   int threads = 0;
   if ((mask & 7) == 5 && hx != 0) {
     const dim3 grid = row_grid(F.ny * C.nz, C.nx, threads);
-    if (hxc != 0)
-      launch(k_prolongate_xz<T, SplitPos>, grid, threads, 0, s, F, x, C, cx, hx,
-             SplitPos{C.ny, hxc});
-    else
-      launch(k_prolongate_xz<T, NaturalPos>, grid, threads, 0, s, F, x, C, cx, hx, NaturalPos());
+    const auto run = [&](auto kernel, auto cpos) {
+      launch(kernel, grid, threads, 0, s, F, x, C, cx, hx, cpos);
+    };
+    if (hxc != 0 && even_only) run(k_prolongate_xz<T, SplitPos, true>, SplitPos{C.ny, hxc});
+    else if (hxc != 0) run(k_prolongate_xz<T, SplitPos, false>, SplitPos{C.ny, hxc});
+    else if (even_only) run(k_prolongate_xz<T, NaturalPos, true>, NaturalPos());
+    else run(k_prolongate_xz<T, NaturalPos, false>, NaturalPos());
     return;
   }
   const dim3 grid = row_grid(F.ny * F.nz, hx == 0 ? F.nx : 2 * hx, threads);
@@ -1871,7 +1877,8 @@ void launch_adjoint_source(cudaStream_t s, int n, const double* dl_dp,
                                           const T*, const Level<T>&, T*, T*, int,  \
                                           int, int, const ZeroStart<T>&);          \
   template void launch_prolongate<T>(cudaStream_t, const Level<T>&, T*,            \
-                                     const Level<T>&, const T*, int, int, int);    \
+                                     const Level<T>&, const T*, int, int, int,     \
+                                     bool);                                        \
   template void launch_mg_enter<T>(cudaStream_t, int, const double*,               \
                                    const uint8_t*, T*, T*, VecLayout,              \
                                    const ZeroStart<T>&);                           \

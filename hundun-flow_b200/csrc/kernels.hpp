@@ -103,11 +103,13 @@ template <class T>
 void launch_defect_restrict(cudaStream_t s, const Level<T>& F, const T* x,
                             const T* b, const Level<T>& C, T* cb, T* cx,
                             int coarsen_mask, int hx, int hxc, const ZeroStart<T>& zero);
-// Fine x in layout hx, coarse x in layout hxc.
+// Fine x in layout hx, coarse x in layout hxc.  even_only: the cells of odd
+// i + k may be left alone, because a y-line colour pass overwrites them before
+// anything reads them (honoured where it saves traffic, in split rows).
 template <class T>
 void launch_prolongate(cudaStream_t s, const Level<T>& F, T* x,
                        const Level<T>& C, const T* cx, int coarsen_mask, int hx = 0,
-                       int hxc = 0);
+                       int hxc = 0, bool even_only = false);
 // ---- zebra line relaxation (kernels_line.cu) --------------------------------
 // Line-colour passes with at least kLinePcrThreshold lines (kLinePcrThresholdLong
 // for lines of kLinePcrLongExtent cells or more) run the chunked-scan solve
