@@ -1,0 +1,36 @@
+"""Transfers with all three axes coarsened (a thread per fine cell in the
+restriction, 2x2x2 fine cells per thread in the prolongation) and the flat
+multigrid entry and exit, bit for bit the C restatement's: rows that end inside,
+at and past a block's 32 coarse cells, odd and even extents per axis, both point
+smoothers, and the residual-minimising exit."""
+import numpy as np
+import pytest
+
+from hfps import workloads
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("oracle_built")]
+
+
+@pytest.mark.parametrize("shape", [(64, 17, 16), (65, 12, 18), (130, 9, 11), (63, 18, 13),
+                                   (12, 40, 33)])
+@pytest.mark.parametrize("smoother", [0, 1])
+def test_point_transfers_match_restatement(cuda_library, shape, smoother):
+    import c_oracle
+    import hfps
+    import ref_oracle
+    s = workloads.make("sphere64", n=shape, seed=6)
+    policy = hfps.Policy.production().replace(point_smoother=smoother, anisotropy_threshold=1e3)
+    mg = ref_oracle.MgPolicy(smoother=smoother, cycle=1, pre=1, post=2, diagonal_shortcut=0.1,
+                             anisotropy_threshold=1e3)
+    r = np.ascontiguousarray(workloads.normals(3, s.cells).reshape(s.rhs.shape))
+    for unit in (1, 0):
+        oracle = c_oracle.OracleSession(s, mg, unit_linear=bool(unit))
+        z = hfps.PressureSolver.from_system(s, policy.replace(unit_linear=unit)) \
+            .apply_preconditioner(r)
+        expected = oracle.apply_mg(r)
+        if unit:
+            assert np.array_equal(z, expected)
+        else:
+            # the scale is a quotient of two sums, added in another order here
+            assert np.linalg.norm(z - expected) <= 4 * np.sqrt(s.cells) * 2.0 ** -53 \
+                * np.linalg.norm(expected)
