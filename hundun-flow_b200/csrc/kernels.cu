@@ -231,12 +231,13 @@ __global__ void k_chebyshev_stage(Level<T> L, const T* __restrict__ x,
                                   const T* __restrict__ b,
                                   T* __restrict__ direction,
                                   T* __restrict__ next, T previous_factor,
-                                  T residual_factor, int first) {
+                                  T residual_factor, int first, int last) {
   grid_dependency_sync();
   const int n = L.nx * L.ny * L.nz;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n;
        c += gridDim.x * blockDim.x)
-    chebyshev_cell<T>(L, x, b, direction, next, previous_factor, residual_factor, first, c);
+    chebyshev_cell<T>(L, x, b, direction, next, previous_factor, residual_factor, first, last,
+                      c);
 }
 
 // Thomas solve of one line (solve_one, src/solver_mg.cpp:3388-3493).
@@ -967,6 +968,85 @@ __global__ void __launch_bounds__(kTileX * kTileY)
   }
   if (finish_reduction<1>(acc, red) && threadIdx.x == 0)
     apply_scalar_op(red.scalars, red.op, acc[0]);
+}
+
+// One Chebyshev stage of a large level over the same tiles: the flat kernel
+// (k_chebyshev_stage) reads x three times and the faces twice through L2, which
+// bounds it there; here each plane comes once.  At 512x256x256 FP32 a pair of
+// stages went from 524 us to 448 (32 and 32 bytes per cell: 161 us each; some of
+// it is the last direction that is no longer stored), at 128^3 from 31.5 to 28.9;
+// below kTiledStageCells the tiles march too few planes each (64^3 FP64 8.4 ->
+// 14.6).
+constexpr long long kTiledStageCells = 1LL << 20;
+
+template <class T, bool FIRST, bool LAST>
+__global__ void __launch_bounds__(kTileX * kTileY)
+    k_chebyshev_tiled(Level<T> L, const T* __restrict__ x, const T* __restrict__ b,
+                      T* __restrict__ direction, T* __restrict__ next, T previous_factor,
+                      T residual_factor, int depth) {
+  grid_dependency_sync();
+  __shared__ T tile[2][kTileY + 2][kTileX + 2];
+  const int nx = L.nx, ny = L.ny, nz = L.nz;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int i = blockIdx.x * kTileX + tx, j = blockIdx.y * kTileY + ty;
+  const int k0 = blockIdx.z * depth, k1 = min(nz, k0 + depth);
+  const bool on = i < nx && j < ny;
+  const int ic = min(i, nx - 1), jc = min(j, ny - 1);
+  const int plane = nx * ny;
+  const unsigned nb = L.neumann;
+  const bool ring_w = tx == 0 && i > 0 && on;
+  const bool ring_e = (tx == kTileX - 1 || i == nx - 1) && i + 1 < nx && on;
+  const bool ring_s = ty == 0 && j > 0 && on;
+  const bool ring_n = (ty == kTileY - 1 || j == ny - 1) && j + 1 < ny && on;
+  int c = ic + nx * (jc + ny * k0);
+  int fxi = face_x_index(L, c, jc, k0), fyi = face_y_index(L, c, k0);
+  T x_prev = k0 > 0 ? x[c - plane] : T(0);
+  T x_cur = x[c];
+  T fz_lo = L.fz[c];
+  int buf = 0;
+  for (int k = k0; k < k1; ++k) {
+    // The plane's coefficients and the next plane of x, in flight before the
+    // barrier.
+    const T x_next = k + 1 < nz ? x[c + plane] : T(0);
+    const T d = L.diag[c], rhs = b[c];
+    const T xl = L.fx[fxi], xh = L.fx[fxi + 1], yl = L.fy[fyi], yh = L.fy[fyi + nx];
+    const T fz_hi = L.fz[c + plane];
+    const T before = FIRST ? T(0) : direction[c];
+    tile[buf][ty + 1][tx + 1] = x_cur;
+    if (ring_w) tile[buf][ty + 1][tx] = x[c - 1];
+    if (ring_e) tile[buf][ty + 1][tx + 2] = x[c + 1];
+    if (ring_s) tile[buf][ty][tx + 1] = x[c - nx];
+    if (ring_n) tile[buf][ty + 2][tx + 1] = x[c + nx];
+    __syncthreads();
+    if (on) {
+      const T xc = x_cur;
+      const T xm = i > 0 ? tile[buf][ty + 1][tx] : ((nb & 1u) ? xc : T(0));
+      const T xp = i + 1 < nx ? tile[buf][ty + 1][tx + 2] : ((nb & 2u) ? xc : T(0));
+      const T ym = j > 0 ? tile[buf][ty][tx + 1] : ((nb & 4u) ? xc : T(0));
+      const T yp = j + 1 < ny ? tile[buf][ty + 2][tx + 1] : ((nb & 8u) ? xc : T(0));
+      const T zm = k > 0 ? x_prev : ((nb & 16u) ? xc : T(0));
+      const T zp = k + 1 < nz ? x_next : ((nb & 32u) ? xc : T(0));
+      T v = d * xc;
+      v -= xl * xm;
+      v -= xh * xp;
+      v -= yl * ym;
+      v -= yh * yp;
+      v -= fz_lo * zm;
+      v -= fz_hi * zp;
+      const T defect = rhs - v;
+      const T scaled = residual_factor * defect / d;
+      const T step = FIRST ? scaled : previous_factor * before + scaled;
+      if (!LAST) direction[c] = step;
+      next[c] = xc + step;
+    }
+    fz_lo = fz_hi;
+    x_prev = x_cur;
+    x_cur = x_next;
+    buf ^= 1;
+    c += plane;
+    fxi += (nx + 1) * ny;
+    fyi += nx * (ny + 1);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1774,9 +1854,29 @@ void launch_rb_color(cudaStream_t s, const Level<T>& L, T* x, const T* b,
 template <class T>
 void launch_chebyshev_stage(cudaStream_t s, const Level<T>& L, const T* x,
                             const T* b, T* direction, T* next,
-                            T previous_factor, T residual_factor, int first) {
-  launch(k_chebyshev_stage<T>, grid_for(HFPS_CELLS(L)), kThreads, 0, s, 
-      L, x, b, direction, next, previous_factor, residual_factor, first);
+                            T previous_factor, T residual_factor, bool first, bool last) {
+  const long long cells = HFPS_CELLS(L);
+  if (cells >= kTiledStageCells) {
+    // Planes per tile as the tiled operator chooses them (tile_depth).
+    int depth = 64;
+    const long long columns = static_cast<long long>((L.nx + kTileX - 1) / kTileX) *
+                              ((L.ny + kTileY - 1) / kTileY);
+    while (depth > 8 && 4 * columns * ((L.nz + depth - 1) / depth) < 3 * 148LL * 8) depth >>= 1;
+    const dim3 grid((L.nx + kTileX - 1) / kTileX, (L.ny + kTileY - 1) / kTileY,
+                    (L.nz + depth - 1) / depth);
+    const dim3 block(kTileX, kTileY);
+    const auto run = [&](auto kernel) {
+      launch(kernel, grid, block, 0, s, L, x, b, direction, next, previous_factor,
+             residual_factor, depth);
+    };
+    if (first && last) run(k_chebyshev_tiled<T, true, true>);
+    else if (first) run(k_chebyshev_tiled<T, true, false>);
+    else if (last) run(k_chebyshev_tiled<T, false, true>);
+    else run(k_chebyshev_tiled<T, false, false>);
+    return;
+  }
+  launch(k_chebyshev_stage<T>, grid_for(cells), kThreads, 0, s, L, x, b, direction, next,
+         previous_factor, residual_factor, first ? 1 : 0, last ? 1 : 0);
 }
 template <class T>
 void launch_defect_restrict(cudaStream_t s, const Level<T>& F, const T* x,
@@ -2147,7 +2247,7 @@ void launch_adjoint_source(cudaStream_t s, int n, const double* dl_dp,
   template void launch_rb_color<T>(cudaStream_t, const Level<T>&, T*, const T*,    \
                                    int);                                           \
   template void launch_chebyshev_stage<T>(cudaStream_t, const Level<T>&, const T*, \
-                                          const T*, T*, T*, T, T, int);            \
+                                          const T*, T*, T*, T, T, bool, bool);     \
   template void launch_defect_restrict<T>(cudaStream_t, const Level<T>&, const T*, \
                                           const T*, const Level<T>&, T*, T*, int,  \
                                           int, int, const ZeroStart<T>&);          \

@@ -84,7 +84,7 @@ void launch_rb_color(cudaStream_t s, const Level<T>& L, T* x, const T* b,
 template <class T>
 void launch_chebyshev_stage(cudaStream_t s, const Level<T>& L, const T* x,
                             const T* b, T* direction, T* next,
-                            T previous_factor, T residual_factor, int first);
+                            T previous_factor, T residual_factor, bool first, bool last);
 // What the producer of a level's rhs b writes to its x: zero, or the first
 // pre-smoothing step from x = 0, which needs no neighbour (the row of a zero
 // x is zero): the first Chebyshev stage x = factor * b / D (also the stage's

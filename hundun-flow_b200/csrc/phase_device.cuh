@@ -191,17 +191,18 @@ __device__ __forceinline__ void rb_slot(const Level<T>& L, T* x, const T* b, int
 
 // One Chebyshev-Jacobi stage at cell c (chebyshev_stream_bulk_kernel,
 // src/solver_mg.cpp:2464-2490): d = f_prev d + f_res (b - A x)/D, x' = x + d.
+// The last stage's direction is not stored: nothing reads it.
 template <class T, class Ld = PlainLoad>
 __device__ __forceinline__ void chebyshev_cell(const Level<T>& L, const T* x, const T* b,
                                                T* direction, T* next, T previous_factor,
-                                               T residual_factor, int first, int c) {
+                                               T residual_factor, int first, int last, int c) {
   int i, j, k;
   cell_coords(c, L.nx, L.ny, i, j, k);
   const T value = row_value<T, Ld>(L, x, i, j, k, c);
   const T defect = Ld::get(b + c) - value;
   const T scaled = residual_factor * defect / L.diag[c];
   const T d = first ? scaled : previous_factor * Ld::get(direction + c) + scaled;
-  direction[c] = d;
+  if (!last) direction[c] = d;
   next[c] = Ld::get(x + c) + d;
 }
 

@@ -825,7 +825,7 @@ void Solver::smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
         if (started && s == 0) continue;
         launch_chebyshev_stage<T>(stream_, view, L.x, L.b, L.r, L.t,
                                   static_cast<T>(previous_factor),
-                                  static_cast<T>(residual_factor), s == 0 ? 1 : 0);
+                                  static_cast<T>(residual_factor), s == 0, s + 1 == sweeps);
         std::swap(L.x, L.t);
       }
     } else {
@@ -2403,7 +2403,7 @@ Status Solver::profile_kernel(int kernel, int repetitions, double* ms,
       return 28.0 / 8.0 * sizeof(T);
     }
     if (L.chebyshev) {
-      launch_chebyshev_stage<T>(stream_, view, L.x, L.b, L.r, L.t, T(0.5), T(0.5), 0);
+      launch_chebyshev_stage<T>(stream_, view, L.x, L.b, L.r, L.t, T(0.5), T(0.5), false, false);
       return 72.0 / 8.0 * sizeof(T);
     }
     launch_rb_color<T>(stream_, view, L.x, L.b, 0);
