@@ -583,7 +583,10 @@ Status Solver::build_hierarchy() {
   }
   coefficients_ready_ = true;
   mixed_ready_ = false;
-  clear_mg_graphs();
+  if (mg_choices() != mg_choices_) {
+    clear_mg_graphs();
+    mg_choices_ = mg_choices();
+  }
   st = check(cudaStreamSynchronize(stream_), "hierarchy");
   if (!st) return st;
   return dic_factor();
@@ -1199,6 +1202,7 @@ void Solver::mg_enqueue(std::vector<DeviceLevel<T>>& levels, const double* r,
   ZeroStart<T> zero = zero_start(levels, 0);
   if (diagonal_shortcut_ || first_sweep_zero_) zero.kind = kZeroNone;
   launch_mg_enter<T>(stream_, n, r, d_active_, L0.b, L0.x, v0, zero);
+  if (capturing_ != nullptr) capturing_->enter = captured_node();
   // MgNullSpace::constant: the rhs, every restricted rhs and the result lose
   // their volume-weighted mean (apply_impl, src/solver_mg.cpp:4900-4960).
   const bool constant = policy_.null_space == HFPS_NULL_SPACE_CONSTANT;
@@ -1224,8 +1228,10 @@ void Solver::mg_enqueue(std::vector<DeviceLevel<T>>& levels, const double* r,
     launch_level_defect<T>(stream_, L0.view(neumann_), L0.x, L0.b, L0.r, L0.split);
     launch_mg_projection<T>(stream_, n, r, d_active_, L0.r,
                             Reduce{d_scalars_, d_partials_, 5});
+    if (capturing_ != nullptr) capturing_->projection = captured_node();
     launch_mg_exit<T>(stream_, n, L0.x, d_active_, &d_scalars_->mg_alpha, z, v0);
   }
+  if (capturing_ != nullptr) capturing_->exit = captured_node();
   for (size_t l = 0; l < levels.size(); ++l) {
     levels[l].x = saved[l].first;
     levels[l].t = saved[l].second;
@@ -1233,9 +1239,60 @@ void Solver::mg_enqueue(std::vector<DeviceLevel<T>>& levels, const double* r,
 }
 
 void Solver::clear_mg_graphs() {
-  for (MgGraph& g : mg_graphs_)
+  for (MgGraph& g : mg_graph_) {
     if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
-  mg_graphs_.clear();
+    if (g.graph != nullptr) cudaGraphDestroy(g.graph);
+    g = MgGraph{};
+  }
+}
+
+// What a coefficient update can change in the kernels of an MG application.
+std::array<int, 8> Solver::mg_choices() const {
+  return {diagonal_shortcut_ ? 1 : 0, coarse_dense_ ? 1 : 0, tail_level_, tail_steps_,
+          tail_blocks_[0], tail_barrier_test_ ? 1 : 0, small_level_, line_ends_ ? 1 : 0};
+}
+
+// The node the last launch on the capturing stream became.
+cudaGraphNode_t Solver::captured_node() const {
+  cudaStreamCaptureStatus status;
+  const cudaGraphNode_t* last = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t count = 0;
+  if (cudaStreamGetCaptureInfo_v3(stream_, &status, nullptr, nullptr, &last, &edges, &count) !=
+          cudaSuccess ||
+      count != 1)
+    return nullptr;
+  return last[0];
+}
+
+// Points the captured application at r and z.  Capturing one graph per pair
+// instead took a solve of FGMRES(12) twelve captures after every coefficient
+// update: 456x256x52, 31 of 163 ms.
+Status Solver::mg_retarget(MgGraph& g, const double* r, double* z) {
+  if (g.r == r && g.z == z) return {};
+  // Argument positions of r and z (-1: none) in a kernel of `count` arguments.
+  const auto set = [&](cudaGraphNode_t node, int count, int r_at, int z_at) -> Status {
+    cudaKernelNodeParams params{};
+    Status st = check(cudaGraphKernelNodeGetParams(node, &params), "graph node");
+    if (!st) return st;
+    void* args[8];
+    for (int a = 0; a < count; ++a) args[a] = params.kernelParams[a];
+    if (r_at >= 0) args[r_at] = &r;
+    if (z_at >= 0) args[z_at] = &z;
+    params.kernelParams = args;
+    return check(cudaGraphExecKernelNodeSetParams(g.exec, node, &params), "graph node update");
+  };
+  Status st = set(g.enter, 7, 1, -1);  // k_mg_enter(n, r, active, b, x, v, zero)
+  if (st && g.projection != nullptr)
+    st = set(g.projection, 5, 1, -1);  // k_mg_projection(n, r_in, active, recursive, red)
+  if (st && policy_.unit_linear && krylov_fusion_)
+    st = set(g.exit, 7, 5, 3);         // k_mg_exit_dot(n, x, active, z, v, r, red)
+  else if (st)
+    st = set(g.exit, 6, -1, 4);        // k_mg_exit(n, x, active, scale_ptr, z, v)
+  if (!st) return st;
+  g.r = r;
+  g.z = z;
+  return {};
 }
 
 Status Solver::mg_apply(bool mixed, const double* r, double* z) {
@@ -1252,28 +1309,34 @@ Status Solver::mg_apply(bool mixed, const double* r, double* z) {
     launches_ += mg_nodes_[slot];
     return check(cudaGetLastError(), "mg launch");
   }
-  cudaGraphExec_t exec = nullptr;
-  for (const MgGraph& g : mg_graphs_)
-    if (g.slot == slot && g.r == r && g.z == z) exec = g.exec;
-  if (exec == nullptr) {
-    cudaGraph_t graph = nullptr;
+  MgGraph& g = mg_graph_[slot];
+  if (g.exec == nullptr) {
+    MgGraph made;
     Status st = check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal),
                       "graph capture begin");
     if (!st) return st;
+    capturing_ = &made;
     if (mixed) mg_enqueue(l32_, r, z);
     else mg_enqueue(l64_, r, z);
-    st = check(cudaStreamEndCapture(stream_, &graph), "graph capture end");
+    capturing_ = nullptr;
+    st = check(cudaStreamEndCapture(stream_, &made.graph), "graph capture end");
     if (!st) return st;
     size_t nodes = 0;
-    cudaGraphGetNodes(graph, nullptr, &nodes);
+    cudaGraphGetNodes(made.graph, nullptr, &nodes);
     mg_nodes_[slot] = nodes;
-    st = check(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
-    cudaGraphDestroy(graph);
-    if (!st) return st;
-    mg_graphs_.push_back(MgGraph{slot, r, z, exec});
+    st = check(cudaGraphInstantiate(&made.exec, made.graph, 0), "graph instantiate");
+    if (!st) {
+      cudaGraphDestroy(made.graph);
+      return st;
+    }
+    made.r = r;
+    made.z = z;
+    g = made;
   }
+  Status st = mg_retarget(g, r, z);
+  if (!st) return st;
   launches_ += mg_nodes_[slot];
-  return check(cudaGraphLaunch(exec, stream_), "graph launch");
+  return check(cudaGraphLaunch(g.exec, stream_), "graph launch");
 }
 
 Status Solver::dic_apply(const double* r, double* z) {
@@ -1282,9 +1345,10 @@ Status Solver::dic_apply(const double* r, double* z) {
   return check(cudaGetLastError(), "IC(0) launch");
 }
 
-Status Solver::precondition(bool mixed) {
-  if (policy_.preconditioner == HFPS_PRECONDITIONER_IC0) return dic_apply(kr_, kz_);
-  return mg_apply(mixed);
+Status Solver::precondition(bool mixed, const double* r, double* z) {
+  if (policy_.preconditioner == HFPS_PRECONDITIONER_IC0)
+    return dic_apply(r != nullptr ? r : kr_, z != nullptr ? z : kz_);
+  return mg_apply(mixed, r, z);
 }
 
 Status Solver::sync_scalars() {
@@ -1487,7 +1551,6 @@ Status Solver::ensure_fgmres_storage(uint32_t restart) {
   if (fg_storage_ != nullptr) {
     Status st = check(cudaStreamSynchronize(stream_), "fgmres storage");
     if (!st) return st;
-    clear_mg_graphs();  // graphs captured on the old basis buffers
     cudaFree(fg_storage_);
     fg_storage_ = nullptr;
   }
@@ -2296,13 +2359,17 @@ Status Solver::apply_preconditioner(const double* r, double* z, int memory,
                                     int precision) {
   if (!coefficients_ready_) return fail(HFPS_INVALID_PLAN, kDetailPlan, "coefficients not set");
   const size_t n = static_cast<size_t>(nx_) * ny_ * nz_;
-  Status st = copy_in(kr_, r, n, memory);
+  // On the caller's arrays where they can be used in place; overlapping ones
+  // go through the staging vectors.
+  const bool in_use = (r + n <= z || z + n <= r) && in_place(r, n, memory) &&
+                      in_place(z, n, memory);
+  Status st;
+  if (!in_use) st = copy_in(kr_, r, n, memory);
   if (!st) return st;
   st = check(cudaMemsetAsync(d_scalars_, 0, sizeof(Scalars), stream_), "scalars");
   if (!st) return st;
-  st = precondition(precision == HFPS_MIXED);
-  if (!st) return st;
-  st = copy_out(z, kz_, n, memory);
+  st = in_use ? precondition(precision == HFPS_MIXED, r, z) : precondition(precision == HFPS_MIXED);
+  if (st && !in_use) st = copy_out(z, kz_, n, memory);
   if (!st) return st;
   return sync_scalars();
 }

@@ -9,6 +9,7 @@
 // device, so an iteration costs one small device-to-host read.
 #pragma once
 
+#include <array>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -99,8 +100,9 @@ class Solver {
   // The MG preconditioner: z = M r, by default on the internal r/z buffers.
   Status mg_apply(bool mixed, const double* r = nullptr, double* z = nullptr);
   void clear_mg_graphs();
-  // z = M r on kr_/kz_ with the policy's preconditioner (MG or cold IC(0)).
-  Status precondition(bool mixed);
+  // z = M r with the policy's preconditioner (MG or cold IC(0)), by default on
+  // kr_/kz_.
+  Status precondition(bool mixed, const double* r = nullptr, double* z = nullptr);
   Status dic_apply(const double* r, double* z);
   Status dic_factor();
   Status krylov_bicgstab(const hfps_control& control, hfps_result& result,
@@ -241,16 +243,26 @@ class Solver {
   double* dic_rows_{};
   double* dic_inv_{};
   double* dic_border_{};      // its sweeps' tickets and tile borders
-  // The MG application captured as one CUDA graph per (precision slot,
-  // input, output) buffers: the PCG uses kr_/kz_, FGMRES every basis
-  // column's V_j/Z_j directly (no copies into fixed buffers).
+  // The MG application captured as one CUDA graph per precision.  Only its
+  // first and last kernels take the caller's r and z, so another pair of
+  // vectors (FGMRES preconditions every basis column in place) is a change of
+  // those nodes' parameters, not another graph; and the graph stays valid
+  // across coefficient updates, which rewrite the same arrays, while the
+  // choices it was captured with (mg_choices) hold.
   struct MgGraph {
-    int slot;
-    const double* r;
-    double* z;
-    cudaGraphExec_t exec;
+    cudaGraph_t graph{};
+    cudaGraphExec_t exec{};
+    // Nodes that take r or z: MG entry, projection (or null), exit.
+    cudaGraphNode_t enter{}, projection{}, exit{};
+    const double* r{};
+    double* z{};
   };
-  std::vector<MgGraph> mg_graphs_;
+  MgGraph mg_graph_[2];
+  MgGraph* capturing_{};      // the graph being captured
+  std::array<int, 8> mg_choices_{};
+  std::array<int, 8> mg_choices() const;
+  Status mg_retarget(MgGraph& g, const double* r, double* z);
+  cudaGraphNode_t captured_node() const;
   size_t mg_nodes_[2]{};      // kernels per MG application (graph nodes)
   uint64_t launches_{};       // kernels launched since the last reset
   bool use_graphs_{true};
