@@ -668,6 +668,28 @@ __global__ void k_coarse_solve(Level<TC> L, T* x, const T* b, TC* xs, TC* bs,
 // thread's loads are issued before its first store.
 constexpr int kFlat = 4;
 
+// Positions of a thread's cells c, c + stride, ... in split rows, the row and x
+// index carried from step to step instead of divided out of c each time.
+struct SplitWalk {
+  int row, i, row_step, i_step;
+  __device__ SplitWalk(const VecLayout& v, int c, int stride) {
+    row = c / v.nx;
+    i = c - row * v.nx;
+    row_step = stride / v.nx;
+    i_step = stride - row_step * v.nx;
+  }
+  __device__ __forceinline__ int next(const VecLayout& v) {
+    const int at = 2 * v.hx * row + (i & 1) * v.hx + (i >> 1);
+    row += row_step;
+    i += i_step;
+    if (i >= v.nx) {
+      i -= v.nx;
+      ++row;
+    }
+    return at;
+  }
+};
+
 template <class T, bool START>
 __global__ void k_mg_enter(int n, const double* __restrict__ r,
                            const uint8_t* __restrict__ active,
@@ -713,15 +735,29 @@ __global__ void k_mg_enter(int n, const double* __restrict__ r,
     }
     return;
   }
-  // A warp per x-row: the split position of a cell is then the row's base
-  // plus its parity half, with no division per cell.
-  for_each_cell_by_rows(v.nx, v.ny, n / (v.nx * v.ny), [&](int i, int j, int k, int c) {
-    const bool on = active == nullptr || active[c] != 0;
-    const int at = 2 * v.hx * (j + v.ny * k) + (i & 1) * v.hx + (i >> 1);
-    const T value = on ? static_cast<T>(r[c]) : T(0);
-    b[at] = value;
-    write_zero_start<START>(zero, value, x, at, (i + j + k) & 1);
-  });
+  // Split rows, where no kernel starts a smoothing step (256^3: a warp per x-row
+  // 64 us, four cells in flight 44; 43 us of bytes).
+  const int stride = gridDim.x * blockDim.x;
+  int c0 = blockIdx.x * blockDim.x + threadIdx.x;
+  SplitWalk walk(v, c0, stride);
+  for (; c0 < n; c0 += kFlat * stride) {
+    double value[kFlat];
+    bool on[kFlat];
+    int at[kFlat];
+#pragma unroll
+    for (int u = 0; u < kFlat; ++u) {
+      at[u] = walk.next(v);
+      const int c = min(c0 + u * stride, n - 1);
+      on[u] = active == nullptr || active[c] != 0;
+      value[u] = r[c];
+    }
+#pragma unroll
+    for (int u = 0; u < kFlat; ++u) {
+      if (c0 + u * stride >= n) break;
+      b[at[u]] = on[u] ? static_cast<T>(value[u]) : T(0);
+      if (zero.kind != kZeroNone) x[at[u]] = T(0);
+    }
+  }
 }
 
 template <class T>
@@ -750,11 +786,25 @@ __global__ void k_mg_exit(int n, const T* __restrict__ x,
     }
     return;
   }
-  for_each_cell_by_rows(v.nx, v.ny, n / (v.nx * v.ny), [&](int i, int j, int k, int c) {
-    const bool on = active == nullptr || active[c] != 0;
-    const int at = 2 * v.hx * (j + v.ny * k) + (i & 1) * v.hx + (i >> 1);
-    z[c] = on ? static_cast<double>(x[at]) * scale : 0.0;
-  });
+  const int stride = gridDim.x * blockDim.x;
+  int c0 = blockIdx.x * blockDim.x + threadIdx.x;
+  SplitWalk walk(v, c0, stride);
+  for (; c0 < n; c0 += kFlat * stride) {
+    T value[kFlat];
+    bool on[kFlat];
+#pragma unroll
+    for (int u = 0; u < kFlat; ++u) {
+      const int at = walk.next(v);
+      const int c = min(c0 + u * stride, n - 1);
+      on[u] = active == nullptr || active[c] != 0;
+      value[u] = x[c0 + u * stride < n ? at : 0];
+    }
+#pragma unroll
+    for (int u = 0; u < kFlat; ++u) {
+      const int c = c0 + u * stride;
+      if (c < n) z[c] = on[u] ? static_cast<double>(value[u]) * scale : 0.0;
+    }
+  }
 }
 
 // MG exit with the PCG's r.z: z = active ? x : 0 (unit scaling) and the sum
@@ -1966,7 +2016,7 @@ void launch_coarse_solve(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
 template <class T>
 void launch_mg_enter(cudaStream_t s, int n, const double* r,
                      const uint8_t* active, T* b, T* x, VecLayout v, const ZeroStart<T>& zero) {
-  const int grid = grid_for(v.hx == 0 ? (n + kFlat - 1) / kFlat : n);
+  const int grid = grid_for((n + kFlat - 1) / kFlat);
   if (zero.kind == kZeroChebyshev || zero.kind == kZeroRedBlack)
     launch(k_mg_enter<T, true>, grid, kThreads, 0, s, n, r, active, b, x, v, zero);
   else
@@ -1975,8 +2025,8 @@ void launch_mg_enter(cudaStream_t s, int n, const double* r,
 template <class T>
 void launch_mg_exit(cudaStream_t s, int n, const T* x, const uint8_t* active,
                     const double* scale_ptr, double* z, VecLayout v) {
-  launch(k_mg_exit<T>, grid_for(v.hx == 0 ? (n + kFlat - 1) / kFlat : n), kThreads, 0, s, n, x,
-         active, scale_ptr, z, v);
+  launch(k_mg_exit<T>, grid_for((n + kFlat - 1) / kFlat), kThreads, 0, s, n, x, active,
+         scale_ptr, z, v);
 }
 template <class T>
 void launch_mg_exit_dot(cudaStream_t s, int n, const T* x, const uint8_t* active, double* z,
