@@ -616,6 +616,79 @@ __global__ void __launch_bounds__(kRowThreads)
     }
 }
 
+// Prolongation and the first post-smoothing step of a small level in one launch
+// (all three axes coarsened, natural order): the first Chebyshev stage, or the
+// red-black colour 1.  A block forms the prolonged x of its 8 x 8 x 4 cells and
+// of a ring around them in shared memory (2.3 values per cell), while the cells'
+// coefficients are on their way, and takes the step from there.  Small levels
+// are bound by launches and latency: 16^3 2.2 + 2.2 -> 3.5 us, and a gap between
+// launches less.  At 64^3 the ring's work shows (8.4 us against 2.6 + 5.0), hence
+// kStepCells.  The result goes to the other x vector, because neighbouring blocks
+// still read the old one.  The same operations per value as the two kernels:
+// bit-identical.
+constexpr int kStepX = 8, kStepY = 8, kStepZ = 4;
+constexpr int kStepThreads = kStepX * kStepY * kStepZ;
+
+template <class T, bool CHEBYSHEV>
+__global__ void __launch_bounds__(kStepThreads)
+    k_prolong_step(Level<T> F, const T* __restrict__ x, const T* __restrict__ b, Level<T> C,
+                   const T* __restrict__ cx, T* __restrict__ direction, T* __restrict__ out,
+                   T factor, int last) {
+  grid_dependency_sync();
+  constexpr int wx = kStepX + 2, wy = kStepY + 2, wz = kStepZ + 2;
+  __shared__ T p[wz][wy][wx];
+  const int nx = F.nx, ny = F.ny, nz = F.nz, plane = nx * ny;
+  const int i0 = blockIdx.x * kStepX, j0 = blockIdx.y * kStepY, k0 = blockIdx.z * kStepZ;
+  const int tid = threadIdx.x;
+  const int tx = tid % kStepX, ty = tid / kStepX % kStepY, tz = tid / (kStepX * kStepY);
+  const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
+  const bool on = i < nx && j < ny && k < nz;
+  const int c = on ? i + nx * (j + ny * k) : 0;
+  const int jc = on ? j : 0, kc = on ? k : 0;
+  const int fxi = face_x_index(F, c, jc, kc), fyi = face_y_index(F, c, kc);
+  const T diag = F.diag[c], rhs = b[c];
+  const T xl = F.fx[fxi], xh = F.fx[fxi + 1], yl = F.fy[fyi], yh = F.fy[fyi + nx];
+  const T zl = F.fz[c], zh = F.fz[c + plane];
+#pragma unroll
+  for (int n = 0; n < (wx * wy * wz + kStepThreads - 1) / kStepThreads; ++n) {
+    const int e = tid + n * kStepThreads;
+    if (e >= wx * wy * wz) break;
+    const int px = e % wx, py = e / wx % wy, pz = e / (wx * wy);
+    const int pi = i0 + px - 1, pj = j0 + py - 1, pk = k0 + pz - 1;
+    T value = T(0);
+    if (pi >= 0 && pi < nx && pj >= 0 && pj < ny && pk >= 0 && pk < nz)
+      value = prolongate_cell<T, PlainLoad, RoLoad, 7>(F, x, C, cx, 7,
+                                                       pi + nx * (pj + ny * pk), pi, pj, pk,
+                                                       pi + nx * (pj + ny * pk));
+    p[pz][py][px] = value;
+  }
+  __syncthreads();
+  if (!on) return;
+  const unsigned nb = F.neumann;
+  const T xc = p[tz + 1][ty + 1][tx + 1];
+  const T xm = i > 0 ? p[tz + 1][ty + 1][tx] : ((nb & 1u) ? xc : T(0));
+  const T xp = i + 1 < nx ? p[tz + 1][ty + 1][tx + 2] : ((nb & 2u) ? xc : T(0));
+  const T ym = j > 0 ? p[tz + 1][ty][tx + 1] : ((nb & 4u) ? xc : T(0));
+  const T yp = j + 1 < ny ? p[tz + 1][ty + 2][tx + 1] : ((nb & 8u) ? xc : T(0));
+  const T zm = k > 0 ? p[tz][ty + 1][tx + 1] : ((nb & 16u) ? xc : T(0));
+  const T zp = k + 1 < nz ? p[tz + 2][ty + 1][tx + 1] : ((nb & 32u) ? xc : T(0));
+  T v = diag * xc;
+  v -= xl * xm;
+  v -= xh * xp;
+  v -= yl * ym;
+  v -= yh * yp;
+  v -= zl * zm;
+  v -= zh * zp;
+  const T defect = rhs - v;
+  if (CHEBYSHEV) {
+    const T d = factor * defect / diag;
+    if (!last) direction[c] = d;
+    out[c] = xc + d;
+  } else {
+    out[c] = ((i + j + k) & 1) != 0 ? xc + T(0.72) * defect / diag : xc;
+  }
+}
+
 // Coarsest level: `sweeps` smoother sweeps in one CTA (mg_cycle coarse
 // branch, src/solver_mg.cpp:4210-4227).  The state is widened to TC (FP64
 // in the mixed-precision hierarchy) for the duration of the solve.
@@ -2014,6 +2087,19 @@ void launch_coarse_solve(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
                                           line_axis);
 }
 template <class T>
+void launch_prolong_step(cudaStream_t s, const Level<T>& F, const T* x, const T* b,
+                         const Level<T>& C, const T* cx, T* direction, T* out, bool chebyshev,
+                         T factor, bool last) {
+  const dim3 grid((F.nx + kStepX - 1) / kStepX, (F.ny + kStepY - 1) / kStepY,
+                  (F.nz + kStepZ - 1) / kStepZ);
+  if (chebyshev)
+    launch(k_prolong_step<T, true>, grid, kStepThreads, 0, s, F, x, b, C, cx, direction, out,
+           factor, last ? 1 : 0);
+  else
+    launch(k_prolong_step<T, false>, grid, kStepThreads, 0, s, F, x, b, C, cx, direction, out,
+           factor, last ? 1 : 0);
+}
+template <class T>
 void launch_mg_enter(cudaStream_t s, int n, const double* r,
                      const uint8_t* active, T* b, T* x, VecLayout v, const ZeroStart<T>& zero) {
   const int grid = grid_for((n + kFlat - 1) / kFlat);
@@ -2307,6 +2393,9 @@ void launch_adjoint_source(cudaStream_t s, int n, const double* dl_dp,
   template void launch_prolongate<T>(cudaStream_t, const Level<T>&, T*,            \
                                      const Level<T>&, const T*, int, int, int,     \
                                      bool);                                        \
+  template void launch_prolong_step<T>(cudaStream_t, const Level<T>&, const T*,    \
+                                       const T*, const Level<T>&, const T*, T*,    \
+                                       T*, bool, T, bool);                         \
   template void launch_mg_enter<T>(cudaStream_t, int, const double*,               \
                                    const uint8_t*, T*, T*, VecLayout,              \
                                    const ZeroStart<T>&);                           \

@@ -110,6 +110,14 @@ template <class T>
 void launch_prolongate(cudaStream_t s, const Level<T>& F, T* x,
                        const Level<T>& C, const T* cx, int coarsen_mask, int hx = 0,
                        int hxc = 0, bool even_only = false);
+// out = x after prolongation of cx and the first post-smoothing step: Chebyshev
+// stage 0 (factor; its direction unless `last`) or red-black colour 1.  All three
+// axes coarsened, natural order, at most kStepCells cells; out must not alias x.
+constexpr long long kStepCells = 1LL << 17;
+template <class T>
+void launch_prolong_step(cudaStream_t s, const Level<T>& F, const T* x, const T* b,
+                         const Level<T>& C, const T* cx, T* direction, T* out, bool chebyshev,
+                         T factor, bool last);
 // ---- zebra line relaxation (kernels_line.cu) --------------------------------
 // Line-colour passes with at least kLinePcrThreshold lines (kLinePcrThresholdLong
 // for lines of kLinePcrLongExtent cells or more) run the chunked-scan solve

@@ -811,14 +811,16 @@ ZeroStart<T> Solver::zero_start(const std::vector<DeviceLevel<T>>& levels, int l
 
 // x_zero: the level's x started from zero (a cycle's first visit).  On point
 // levels its first step is then already taken (zero_start); the chunked scan
-// uses it to skip reading x in the first sweep.
+// uses it to skip reading x in the first sweep.  first_done: the caller took
+// the first step of a point level (launch_prolong_step).
 template <class T>
 void Solver::smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
-                    bool reverse, bool x_zero) {
+                    bool reverse, bool x_zero, bool first_done) {
   DeviceLevel<T>& L = levels[level];
   const Level<T> view = L.view(neumann_);
   if (L.line_mask == 0) {
-    const bool started = x_zero && policy_.null_space == HFPS_NULL_SPACE_NONE;
+    const bool started =
+        first_done || (x_zero && policy_.null_space == HFPS_NULL_SPACE_NONE);
     if (L.chebyshev) {
       // The ping-pong partner becomes the solution after odd stage counts.
       ChebyshevStages stages(policy_.chebyshev_lower_spectrum_fraction);
@@ -1143,7 +1145,7 @@ void Solver::cycle(std::vector<DeviceLevel<T>>& levels, int level, int counter,
   }
   DeviceLevel<T>& F = levels[level];
   DeviceLevel<T>& C = levels[level + 1];
-  smooth(levels, level, policy_.pre_sweeps, false, x_zero);
+  smooth(levels, level, policy_.pre_sweeps, false, x_zero, false);
   // Retained defect + restrict_residual in one pass.
   launch_defect_restrict<T>(stream_, F.view(neumann_), F.x, F.b, C.view(neumann_),
                             C.b, C.x, F.coarsen_mask, F.split, C.split,
@@ -1180,11 +1182,20 @@ void Solver::cycle(std::vector<DeviceLevel<T>>& levels, int level, int counter,
     cycle(levels, level + 1, counter, true);
     if (counter > 1) cycle(levels, level + 1, counter - 1, false);
   }
+  if (F.line_mask == 0 && F.coarsen_mask == 7 && C.split == 0 && F.cells() <= kStepCells) {
+    double unused, residual;
+    ChebyshevStages(policy_.chebyshev_lower_spectrum_fraction).next(unused, residual);
+    launch_prolong_step<T>(stream_, F.view(neumann_), F.x, F.b, C.view(neumann_), C.x, F.r, F.t,
+                           F.chebyshev, static_cast<T>(residual), policy_.post_sweeps == 1);
+    std::swap(F.x, F.t);
+    smooth(levels, level, policy_.post_sweeps, true, false, true);
+    return;
+  }
   // The way up starts with colour 1 (reverse order), which without end terms
   // reads only colour 0: half the prolongation (256^3 level 0 66 -> 44 us).
   launch_prolongate<T>(stream_, F.view(neumann_), F.x, C.view(neumann_), C.x,
                        F.coarsen_mask, F.split, C.split, F.line_mask == 2 && !line_ends_);
-  smooth(levels, level, policy_.post_sweeps, true, false);
+  smooth(levels, level, policy_.post_sweeps, true, false, false);
 }
 
 // NativeCartesianMgPlan::apply_impl (src/solver_mg.cpp:4814-5122).

@@ -114,7 +114,7 @@ class Solver {
   void cycle(std::vector<DeviceLevel<T>>& levels, int level, int counter, bool x_zero);
   template <class T>
   void smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
-              bool reverse, bool x_zero);
+              bool reverse, bool x_zero, bool first_done);
   template <class T>
   void coarse_solve(std::vector<DeviceLevel<T>>& levels, bool x_zero);
   // What the producer of `level`'s rhs writes to its x (ZeroKind).

@@ -34,3 +34,24 @@ def test_point_transfers_match_restatement(cuda_library, shape, smoother):
             # the scale is a quotient of two sums, added in another order here
             assert np.linalg.norm(z - expected) <= 4 * np.sqrt(s.cells) * 2.0 ** -53 \
                 * np.linalg.norm(expected)
+
+
+@pytest.mark.parametrize("shape,post", [((9, 9, 9), 1), ((33, 18, 21), 1), ((48, 50, 54), 3),
+                                        ((51, 51, 52), 1)])
+@pytest.mark.parametrize("smoother", [0, 1])
+def test_prolongation_with_first_step_matches_restatement(cuda_library, shape, post, smoother):
+    """One and three post-smoothing steps (the first of them taken with the
+    prolongation up to 2^17 cells), cells at, inside and past a block's 8 x 8 x 4,
+    and a grid just above that size."""
+    import c_oracle
+    import hfps
+    import ref_oracle
+    s = workloads.make("sphere64", n=shape, seed=6)
+    policy = hfps.Policy.production().replace(point_smoother=smoother, post_sweeps=post,
+                                              anisotropy_threshold=1e3)
+    mg = ref_oracle.MgPolicy(smoother=smoother, cycle=1, pre=1, post=post, diagonal_shortcut=0.1,
+                             anisotropy_threshold=1e3)
+    r = np.ascontiguousarray(workloads.normals(3, s.cells).reshape(s.rhs.shape))
+    z = hfps.PressureSolver.from_system(s, policy).apply_preconditioner(r)
+    oracle = c_oracle.OracleSession(s, mg, unit_linear=True)
+    assert np.array_equal(z, oracle.apply_mg(r))
