@@ -66,6 +66,26 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
 #endif
 }
 
+// Launch of `blocks` CTAs (at most 8, the portable size) as one cluster.
+template <class... Params, class... Args>
+inline void launch_cluster(void (*kernel)(Params...), int blocks, dim3 block, size_t smem,
+                           cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = blocks;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = HFPS_USE_PDL ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // Bit f of `neumann` is set when face f (x-,x+,y-,y+,z-,z+) is Neumann; a
 // clear bit is Dirichlet (neighbour value 0).  Neumann reads the cell
 // itself (MgPointBoundaryMode::self, src/solver_mg.cpp:940-963).

@@ -164,6 +164,11 @@ void launch_line_pass(cudaStream_t s, const Level<T>& L, T* x, const T* b,
 // kCoarseColumnsOn applies the sweeps to columns already there (a further
 // axis after the first).
 enum CoarseColumns : int { kCoarseVector = 0, kCoarseColumns = 1, kCoarseColumnsOn = 2 };
+// All `passes` colour passes of one axis, starting with colour `first`, in one
+// launch.  False: not launched, the level is not a small PCR level.
+template <class T>
+bool launch_line_sweeps(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* fac,
+                        int axis, int first, int passes);
 template <class T, class TC>
 bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
                         const TC* fac, int sweeps, int axis, int columns = kCoarseVector);

@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(TailProgram<T> prog) {
   constexpr int G = kTailThreads / P;  // lines a CTA relaxes at once
   static_assert(kTailThreads / 32 == kDenseWarps, "dense map grouping");
   extern __shared__ double tail_smem[];
-  T* sd = reinterpret_cast<T*>(tail_smem);                  // PCR line values, G x P
-  double* v = tail_smem + kTailThreads;                      // dense map: x then b
+  T* sd = reinterpret_cast<T*>(tail_smem);                  // PCR line values, G x 2 x P
+  double* v = tail_smem + 2 * kTailThreads;                    // dense map: x then b
   double* part = v + 2 * prog.dense_n;                       // dense map partials
   const unsigned blocks = gridDim.x;
   const int tid = threadIdx.x;
@@ -94,10 +94,12 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(TailProgram<T> prog) {
         const int lines = ((a_extent + 1) >> 1) * b_extent;
         // The trip count depends on the CTA only: every thread reaches the
         // barriers inside pcr_line_slot; slots past the last line write nothing.
-        for (int t0 = blockIdx.x * G; t0 < lines; t0 += blocks * G)
+        for (int t0 = blockIdx.x * G; t0 < lines; t0 += blocks * G) {
           pcr_line_slot<T, STEPS>(L, static_cast<T*>(op.p0), static_cast<const T*>(op.p1),
                                   static_cast<const T*>(op.p2), axis, op.arg, t0 + g, s,
-                                  sd + g * P);
+                                  sd + g * 2 * P, [] {});
+          __syncthreads();
+        }
         break;
       }
       case kTailRestrict: {
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(TailProgram<T> prog) {
 
 template <class T, int STEPS>
 size_t tail_smem_bytes(int dense_n) {
-  return (2 * static_cast<size_t>(kTailThreads) + 2 * static_cast<size_t>(dense_n)) *
+  return (3 * static_cast<size_t>(kTailThreads) + 2 * static_cast<size_t>(dense_n)) *
          sizeof(double);
 }
 

@@ -104,24 +104,36 @@ __device__ __forceinline__ void pcr_load(const T* __restrict__ fac, size_t slab,
   for (int e = 0; e <= 2 * STEPS; ++e) r.k[e] = fac[e * slab + at];
 }
 
-// PCR right-hand-side elimination with register-held factors; returns x_s.
-// sd is written by the other threads of the line between barriers, so it
-// must not be __restrict__-qualified.
+// PCR right-hand-side elimination of d with register-held factors; returns x_s.
+// Lines of at most 32 rows lie within a warp and exchange values by shuffles.  For
+// longer ones sd holds 2 * 2^STEPS values, a step writing the half that the step
+// before did not read, so one barrier per step is enough (with two barriers a step
+// everywhere 60 lines of 16 rows took 3.35 us a pass, now 3.16; 8 of 256 rows 3.45,
+// now 3.18).  The last step reads half (STEPS - 1) % 2: a caller that goes on to
+// another line synchronises first.
 template <class T, int STEPS>
-__device__ __forceinline__ T pcr_apply(const PcrRow<T, STEPS>& r, T* sd, int s) {
+__device__ __forceinline__ T pcr_apply(const PcrRow<T, STEPS>& r, T* sd, int s, T d) {
   constexpr int P = 1 << STEPS;
 #pragma unroll
   for (int step = 0; step < STEPS; ++step) {
     const int h = 1 << step;
     const int lo = s - h, hi = s + h;
-    const T dlo = lo >= 0 ? sd[lo] : T(0);
-    const T dhi = hi < P ? sd[hi] : T(0);
-    const T nd = sd[s] - dlo * r.k[2 * step] - dhi * r.k[2 * step + 1];
-    __syncthreads();
-    sd[s] = nd;
-    __syncthreads();
+    T dlo, dhi;
+    if constexpr (STEPS <= 5) {
+      dlo = __shfl_up_sync(~0u, d, h, P);
+      dhi = __shfl_down_sync(~0u, d, h, P);
+    } else {
+      T* now = sd + (step & 1) * P;
+      now[s] = d;
+      __syncthreads();
+      dlo = now[max(lo, 0)];
+      dhi = now[min(hi, P - 1)];
+    }
+    dlo = lo >= 0 ? dlo : T(0);
+    dhi = hi < P ? dhi : T(0);
+    d = d - dlo * r.k[2 * step] - dhi * r.k[2 * step + 1];
   }
-  return sd[s] / r.k[2 * STEPS];
+  return d / r.k[2 * STEPS];
 }
 
 template <class T, class Ld = PlainLoad>
@@ -135,13 +147,14 @@ __device__ __forceinline__ T line_rhs_any(const Level<T>& L, const T* x,
 
 
 // One line slot of a zebra colour pass with PCR (k_line_pcr_factored_color):
-// line t of colour `color`, row s of P = 2^STEPS threads, sd the slot's P
+// line t of colour `color`, row s of P = 2^STEPS threads, sd the slot's 2 * P
 // shared-memory values.  Every thread of the CTA calls it (it synchronises
-// the CTA); slots past the colour's lines do no memory writes.
-template <class T, int STEPS, class Ld = PlainLoad>
+// the CTA, pcr_apply); slots past the colour's lines do no memory writes.  `ready` runs
+// between the loads of the factors and the first read of x and rhs.
+template <class T, int STEPS, class Ld = PlainLoad, class Ready>
 __device__ __forceinline__ void pcr_line_slot(const Level<T>& L, T* x, const T* rhs,
                                               const T* __restrict__ fac, int axis,
-                                              int color, int t, int s, T* sd) {
+                                              int color, int t, int s, T* sd, Ready ready) {
   constexpr int P = 1 << STEPS;
   const int a_extent = axis == 0 ? L.ny : L.nx;
   const int b_extent = axis == 2 ? L.ny : L.nz;
@@ -154,6 +167,7 @@ __device__ __forceinline__ void pcr_line_slot(const Level<T>& L, T* x, const T* 
   const size_t at = static_cast<size_t>(valid ? fa + a_extent * fb : 0) * P + s;
   PcrRow<T, STEPS> r;
   pcr_load(fac, slab, at, r);
+  ready();
   int c = 0;
   T d = T(0);
   if (valid && s < extent) {
@@ -162,9 +176,7 @@ __device__ __forceinline__ void pcr_line_slot(const Level<T>& L, T* x, const T* 
     c = i + L.nx * (j + L.ny * k);
     d = line_rhs_any<T, Ld>(L, x, rhs, axis, fa, fb, s, extent, c);
   }
-  sd[s] = d;
-  __syncthreads();
-  const T value = pcr_apply(r, sd, s);
+  const T value = pcr_apply(r, sd, s, d);
   if (valid && s < extent) x[c] = value;
 }
 

@@ -850,6 +850,8 @@ void Solver::smooth(std::vector<DeviceLevel<T>>& levels, int level, int sweeps,
   const bool one_axis = (L.line_mask & (L.line_mask - 1)) == 0;
   const auto run_axis = [&](int axis) {
     const int first = reverse ? 1 : 0;
+    if (launch_line_sweeps<T>(stream_, view, L.x, L.b, L.lfac[axis], axis, first, 2 * sweeps))
+      return;
     for (int s = 0; s < sweeps; ++s)
       for (int pass = 0; pass < 2; ++pass) {
         const bool fresh = x_zero && one_axis && s == 0;

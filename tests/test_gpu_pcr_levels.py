@@ -1,0 +1,54 @@
+"""Line levels relaxed with PCR, against the C restatement's zebra order: rows of
+every power of two up to 256 and just past one, exchanged within a warp (up to 32
+rows) and across warps, and numbers of lines at and past what one cluster launch
+of all passes holds, along each axis.  The bars are those of the line relaxation:
+1e-11 relative in FP64 (exact eliminations in another order), and in FP32 the
+unit roundoff times the condition of a line, up to the square of its cells."""
+import numpy as np
+import pytest
+
+from hfps import workloads
+from test_gpu_parity import stretched_front
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("oracle_built")]
+
+CASES = [
+    # line axis, rows, the other two extents (lower axis first)
+    (1, 16, (16, 16)),    # 128 lines a colour: 8 CTAs of 16
+    (1, 16, (17, 16)),    # 144: separate passes
+    (1, 17, (16, 8)),     # 64 lines of 32 threads
+    (1, 32, (9, 15)),     # separate passes
+    (1, 33, (8, 8)),      # first with shared memory
+    (1, 64, (7, 9)),
+    (1, 129, (4, 4)),
+    (1, 256, (4, 4)),
+    (1, 256, (4, 5)),     # separate passes
+    (0, 30, (11, 10)),
+    (0, 100, (6, 5)),
+    (2, 24, (12, 9)),
+    (2, 65, (5, 6)),
+]
+
+
+@pytest.mark.parametrize("axis,rows,others", CASES)
+@pytest.mark.parametrize("pre,post", [(1, 2), (3, 1)])
+def test_pcr_levels_match_restatement(cuda_library, axis, rows, others, pre, post):
+    import c_oracle
+    import hfps
+    import ref_oracle
+    shape = list(others)
+    shape.insert(axis, rows)
+    s = stretched_front(tuple(shape), axis, 1.0 + 3.0 / rows)
+    policy = hfps.Policy.production().replace(pre_sweeps=pre, post_sweeps=post,
+                                              anisotropy_threshold=4.0)
+    g = hfps.PressureSolver.from_system(s, policy)
+    assert g.levels()[0][3] == 1 << axis
+    oracle = c_oracle.OracleSession(
+        s, ref_oracle.MgPolicy(smoother=1, cycle=1, pre=pre, post=post, diagonal_shortcut=0.1,
+                               anisotropy_threshold=4.0), unit_linear=True, line_order=1)
+    r = np.ascontiguousarray(workloads.normals(3, s.cells).reshape(s.rhs.shape))
+    expected = oracle.apply_mg(r)
+    size = np.linalg.norm(expected)
+    assert np.linalg.norm(g.apply_preconditioner(r) - expected) <= 1e-11 * size
+    mixed = g.apply_preconditioner(r, precision=hfps.MIXED)
+    assert np.linalg.norm(mixed - expected) <= max(shape) ** 2 * 2.0 ** -24 * size
