@@ -821,7 +821,9 @@ ScanShape scan_shape(long long per_color, int extent) {
 // half-used sectors cost more than it gives (456x256x52 y-lines 65.6 -> 71 us),
 // and levels that three blocks per SM hold anyway gain nothing (64x256x64 9.9 ->
 // 11.0 us, 32x256x32 7.3 -> 8.3): those keep the kernel with the end terms,
-// which are exact zeros then.
+// which are exact zeros then.  FP32 has 64 registers and two blocks per SM either
+// way, and its level-0 pass is slower without them (94.5 -> 100.3 us), but for the
+// fresh one, which then reads nothing but rhs.
 struct ScanFlags {
   int hx;
   bool zero_other, zero_self, ends;
@@ -835,9 +837,9 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
   const dim3 block(LPB, sh.chunks);
   // Without end terms the zero flag is an argument of the ordinary kernel (a
   // kernel of its own takes more registers); with them it is a mode.
-  const bool ends = f.ends || f.hx == 0 || blocks <= 3 * 148;
-  const int mode = f.zero_other && f.zero_self ? kScanFresh
-                                               : (f.zero_self && ends ? kScanOwnZero : kScanNormal);
+  const bool fresh = f.zero_other && f.zero_self;
+  const bool ends = f.ends || f.hx == 0 || blocks <= 3 * 148 || (sizeof(T) == 4 && !fresh);
+  const int mode = fresh ? kScanFresh : (f.zero_self && ends ? kScanOwnZero : kScanNormal);
   const bool split = f.hx != 0;
 #define HFPS_SCAN_RUN(MODE, SPLIT, ENDS)                                                    \
   launch(k_line_scan_color<T, AXIS, LPB, MODE, SPLIT, ENDS>, blocks, block, smem, s, L, x, b, \
