@@ -44,6 +44,17 @@ __device__ __forceinline__ void grid_dependency_sync() {
 #endif
 }
 
+// Lets `kernel` be launched with `smem` bytes of dynamic shared memory, at most
+// `largest`.  The limit belongs to the process: it is always set to the kernel's
+// largest, never to what one launch needs, or a handle on another thread could
+// lower it between this call and the launch.
+template <class... Params>
+inline void allow_shared(void (*kernel)(Params...), size_t smem, size_t largest) {
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(largest));
+}
+
 // Launches kernel<<<grid, block, smem, stream>>>(args...) with programmatic
 // stream serialisation allowed.
 template <class... Params, class... Args>

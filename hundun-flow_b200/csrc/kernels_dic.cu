@@ -265,8 +265,7 @@ void launch_sweep(cudaStream_t s, const Level<double>& L, const double* in, doub
   constexpr int arrays = MODE == kDicPivots ? 4 : 5;
   constexpr size_t smem =
       (2 * arrays * kDicColumns * kDicPitch + 2 * kDicChunk * kDicValues) * sizeof(double);
-  cudaFuncSetAttribute(k_dic_sweep<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(smem));
+  allow_shared(k_dic_sweep<MODE>, smem, smem);
   launch(k_dic_sweep<MODE>, dic_tiles(L.ny, L.nz), kDicThreads, smem, s, L, in, out, inv, border,
          scalars, (L.ny + kDicY - 1) / kDicY, (L.nz + kDicZ - 1) / kDicZ);
 }

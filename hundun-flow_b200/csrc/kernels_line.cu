@@ -880,12 +880,10 @@ void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T*
   sh.lines = threads / sh.chunks;
   while (sh.lines > threads / 32 && per_color < 592LL * sh.lines)
     sh.lines = std::max(threads / 32, sh.lines / 2);
-  const int arrays = 1 + ScanConfig<T>::arrays;
-  const size_t smem = static_cast<size_t>(sh.lines) * sh.chunks *
-                      (static_cast<size_t>(arrays) * sh.pitch + 4) * sizeof(T);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_line_scan_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(smem));
+  constexpr size_t arrays = 1 + ScanConfig<T>::arrays;
+  const size_t smem =
+      static_cast<size_t>(sh.lines) * sh.chunks * (arrays * sh.pitch + 4) * sizeof(T);
+  allow_shared(k_line_scan_x<T>, smem, threads * (arrays * (rows | 1) + 4) * sizeof(T));
   launch(k_line_scan_x<T>, static_cast<int>((per_color + sh.lines - 1) / sh.lines), threads, smem,
          s, L, x, b, fac, color, sh);
 }
@@ -1039,16 +1037,15 @@ bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
   if (P > 512) return false;
   lpb = std::max(1, std::min({512 / P, 4, ((a_extent + 1) / 2) * b_extent}));
   const size_t cells = static_cast<size_t>(L.nx) * L.ny * L.nz;
-  if ((2 * cells + static_cast<size_t>(P) * lpb) * sizeof(TC) > 200 * 1024) return false;
+  constexpr size_t kCoarseLineShared = 200 * 1024;
+  if ((2 * cells + static_cast<size_t>(P) * lpb) * sizeof(TC) > kCoarseLineShared) return false;
   const size_t smem = (2 * cells + static_cast<size_t>(2) * P * lpb) * sizeof(TC);
   const dim3 block(P, lpb);
   switch (steps) {
 #define HFPS_COARSE_CASE(N)                                                      \
   case N:                                                                        \
-    if (smem > 48 * 1024)                                                        \
-      cudaFuncSetAttribute(k_coarse_line_smem<T, TC, N>,                         \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,          \
-                           static_cast<int>(smem));                              \
+    allow_shared(k_coarse_line_smem<T, TC, N>, smem,                             \
+                 kCoarseLineShared + 512 * sizeof(TC));                          \
     launch(k_coarse_line_smem<T, TC, N>,                                          \
            columns != kCoarseVector ? 2 * static_cast<int>(cells) : 1, block, smem, s, L, x, \
            b, fac, sweeps, axis, columns);                                         \
@@ -1107,10 +1104,9 @@ __global__ void __launch_bounds__(32 * kDenseWarps)
 template <class T>
 void launch_coarse_dense(cudaStream_t s, int n, const double* op, const T* x,
                          const T* b, T* out, bool x_zero) {
+  static_assert((2 * kCoarseDenseMaxCells + 32 * kDenseWarps) * sizeof(double) <= 48 * 1024,
+                "default shared memory limit");
   const size_t smem = (2 * static_cast<size_t>(n) + 32 * kDenseWarps) * sizeof(double);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_coarse_dense<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(smem));
   launch(k_coarse_dense<T>, (n + 31) / 32, dim3(32, kDenseWarps), smem, s, n, op, x, b, out,
          x_zero);
 }

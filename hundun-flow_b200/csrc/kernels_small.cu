@@ -396,9 +396,7 @@ template <class T>
 bool launch_small_cycle(cudaStream_t s, SmallProgram<T>& prog) {
   const size_t smem = small_layout(prog);
   if (smem > kSmallMaxShared) return false;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_small_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(smem));
+  allow_shared(k_small_cycle<T>, smem, kSmallMaxShared);
   launch(k_small_cycle<T>, 1, kSmallThreads, smem, s, prog);
   return true;
 }

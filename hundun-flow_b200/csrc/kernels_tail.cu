@@ -164,9 +164,7 @@ size_t tail_smem_bytes(int dense_n) {
 template <class T, int STEPS>
 int tail_blocks_per_sm(int dense_n) {
   const size_t smem = tail_smem_bytes<T, STEPS>(dense_n);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_tail<T, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(smem));
+  allow_shared(k_tail<T, STEPS>, smem, tail_smem_bytes<T, STEPS>(kCoarseDenseMaxCells));
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tail<T, STEPS>, kTailThreads,
                                                     smem) != cudaSuccess) {

@@ -1,0 +1,86 @@
+"""Host paths of the library that no GPU run reaches: calls that the CUDA
+runtime refuses, and what several handles in one process do to one another.
+The library runs here on a stand-in for the runtime (fake_cudart.cpp), each
+case in a process of its own; kernels do not run, so no result is looked at."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_INCLUDE = "/usr/local/cuda/include"
+
+PREAMBLE = """
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, {package!r})
+import hfps
+fake = ctypes.CDLL({fake!r})
+fake.fake_entry_argument.restype = ctypes.c_void_p
+
+def solver(shape, stretch=None, **policy):
+    faces = []
+    for axis, n in enumerate(shape):
+        w = (1.0 + 5.0 / n if axis == stretch else 1.0) ** np.arange(n)
+        faces.append(np.concatenate([[0.0], np.cumsum(w * n / w.sum())]))
+    policy.setdefault("anisotropy_threshold", 1e9 if stretch is None else 4.0)
+    s = hfps.PressureSolver(shape, faces, (1, 0, 1, 1, 1, 1), None,
+                            hfps.Policy.production().replace(**policy))
+    update(s)
+    return s
+
+def update(s):
+    s.set_coefficients(np.ones(s.cells), *(np.ones(n) for n in s.face_counts))
+
+def apply(s, r=None, precision=hfps.FP64, z=None):
+    r = np.ones(s.cells) if r is None else r
+    z = np.empty(s.cells) if z is None else z
+    s._check(s._lib.hfps_apply_preconditioner(s._handle, r.ctypes.data, z.ctypes.data,
+                                              hfps.DEVICE, precision), "apply")
+
+def refused(call):
+    try:
+        call()
+    except hfps.SolverError as e:
+        return str(e)
+    return ""
+"""
+
+
+@pytest.fixture(scope="module")
+def run(cuda_library, tmp_path_factory):
+    if not os.path.isdir(CUDA_INCLUDE):
+        pytest.skip("CUDA headers not installed")
+    fake = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{CUDA_INCLUDE}",
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", fake], check=True)
+    preamble = PREAMBLE.format(package=os.path.dirname(cuda_library), fake=fake)
+
+    def run(body):
+        proc = subprocess.run([sys.executable, "-c", preamble + textwrap.dedent(body)],
+                              env=dict(os.environ, LD_PRELOAD=fake), capture_output=True,
+                              text=True, timeout=300)
+        assert proc.returncode == 0, proc.stdout + proc.stderr
+    return run
+
+
+@pytest.mark.parametrize("first,second,stretch", [
+    ((40, 40, 40), (72, 72, 72), None),    # one-CTA point levels: 86,112 and 67,248 bytes
+    ((512, 40, 40), (600, 40, 40), 0),     # x-line scan: 56,320 and 50,160
+    ((40, 500, 40), (40, 450, 40), 1),     # sweeps of a coarsest level of y-lines
+])
+def test_shared_memory_limits_hold_for_every_handle(run, first, second, stretch):
+    """A kernel's limit belongs to the process: a second handle, whose launches
+    need less, must not take it below what the first one's need."""
+    run(f"""
+    a = solver({first}, {stretch})
+    b = solver({second}, {stretch})
+    for s in (a, b, a):
+        for precision in (hfps.FP64, hfps.MIXED):
+            apply(s, precision=precision)
+        update(s)
+    assert fake.fake_calls(b"cudaFuncSetAttribute") > 0
+    assert fake.fake_lowered() == 0
+    """)
