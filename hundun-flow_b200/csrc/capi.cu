@@ -28,7 +28,10 @@ template <class F>
 int guarded(hfps_solver* s, F&& body) {
   if (s == nullptr || s->impl == nullptr) return HFPS_INVALID_PLAN;
   try {
-    return finish(s, body(*s->impl));
+    hfps::Status st = body(*s->impl);
+    if (st) st = s->impl->launched("kernel launch");
+    else hfps::take_launch_error();  // the next call starts clean
+    return finish(s, st);
   } catch (const std::bad_alloc&) {
     s->error = "host allocation failure";
     return HFPS_ALLOCATION_FAILURE;

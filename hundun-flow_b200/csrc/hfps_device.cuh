@@ -55,6 +55,24 @@ inline void allow_shared(void (*kernel)(Params...), size_t smem, size_t largest)
                          static_cast<int>(largest));
 }
 
+// The calling thread's first refused launch since take_launch_error was last
+// asked.  The runtime's own record is cleared, so it does not surface in the
+// caller's code.
+inline cudaError_t& launch_error() {
+  static thread_local cudaError_t error = cudaSuccess;
+  return error;
+}
+inline void note_launch(cudaError_t e) {
+  if (e == cudaSuccess) return;
+  cudaGetLastError();
+  if (launch_error() == cudaSuccess) launch_error() = e;
+}
+inline cudaError_t take_launch_error() {
+  const cudaError_t e = launch_error();
+  launch_error() = cudaSuccess;
+  return e;
+}
+
 // Launches kernel<<<grid, block, smem, stream>>>(args...) with programmatic
 // stream serialisation allowed.
 template <class... Params, class... Args>
@@ -71,9 +89,10 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  note_launch(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
 #else
   kernel<<<grid, block, smem, stream>>>(static_cast<Params>(args)...);
+  note_launch(cudaPeekAtLastError());
 #endif
 }
 
@@ -94,7 +113,7 @@ inline void launch_cluster(void (*kernel)(Params...), int blocks, dim3 block, si
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = HFPS_USE_PDL ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  note_launch(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
 }
 
 // Bit f of `neumann` is set when face f (x-,x+,y-,y+,z-,z+) is Neumann; a

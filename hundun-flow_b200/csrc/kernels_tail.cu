@@ -187,7 +187,9 @@ bool launch_tail_steps(cudaStream_t s, const TailProgram<T>& prog, int blocks) {
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_tail<T, STEPS>, prog) == cudaSuccess;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_tail<T, STEPS>, prog);
+  note_launch(e);
+  return e == cudaSuccess;
 }
 
 }  // namespace

@@ -122,6 +122,8 @@ Status Solver::check(cudaError_t e, const char* what) {
                 kDetailCuda};
 }
 
+Status Solver::launched(const char* what) { return check(take_launch_error(), what); }
+
 Solver::~Solver() {
   if (stream_ != nullptr) cudaStreamSynchronize(stream_);
   clear_mg_graphs();
@@ -530,7 +532,7 @@ Status Solver::build_hierarchy() {
       columns = kCoarseColumnsOn;
     }
   }
-  Status st = check(cudaGetLastError(), "hierarchy kernels");
+  Status st = launched("hierarchy kernels");
   if (!st) return st;
   select_tail();
   select_small();
@@ -626,8 +628,9 @@ Status Solver::refresh_mixed() {
   for (auto& L : l32_)
     for (int a = 0; a < 3; ++a)
       if (L.lfac[a] != nullptr) launch_line_factors<float>(stream_, L.view(neumann_), a, L.lfac[a]);
-  mixed_ready_ = true;
-  return check(cudaGetLastError(), "mixed conversion");
+  const Status st = launched("mixed conversion");
+  mixed_ready_ = bool(st);
+  return st;
 }
 
 Status Solver::set_coefficients(const double* diag, const double* fx,
@@ -1320,7 +1323,7 @@ Status Solver::mg_apply(bool mixed, const double* r, double* z) {
     if (mixed) mg_enqueue(l32_, r, z);
     else mg_enqueue(l64_, r, z);
     launches_ += mg_nodes_[slot];
-    return check(cudaGetLastError(), "mg launch");
+    return launched("mg launch");
   }
   MgGraph& g = mg_graph_[slot];
   if (g.exec == nullptr) {
@@ -1332,7 +1335,11 @@ Status Solver::mg_apply(bool mixed, const double* r, double* z) {
     if (mixed) mg_enqueue(l32_, r, z);
     else mg_enqueue(l64_, r, z);
     capturing_ = nullptr;
+    // A graph that lacks a refused kernel must not be kept.
+    const Status complete = launched("graph capture");
     st = check(cudaStreamEndCapture(stream_, &made.graph), "graph capture end");
+    if (st && !complete) cudaGraphDestroy(made.graph);
+    if (!complete) return complete;
     if (!st) return st;
     size_t nodes = 0;
     cudaGraphGetNodes(made.graph, nullptr, &nodes);
@@ -1355,7 +1362,7 @@ Status Solver::mg_apply(bool mixed, const double* r, double* z) {
 Status Solver::dic_apply(const double* r, double* z) {
   launch_dic_apply(stream_, l64_[0].view(neumann_), r, z, dic_inv_, dic_border_, d_scalars_);
   launches_ += 2;
-  return check(cudaGetLastError(), "IC(0) launch");
+  return launched("IC(0) launch");
 }
 
 Status Solver::precondition(bool mixed, const double* r, double* z) {
@@ -1374,8 +1381,11 @@ Status Solver::sync_scalars() {
   return wait_status();
 }
 
-// Waits between blocks that ran out (the scalars are on the host).
+// A refused launch, or waits between blocks that ran out (the scalars are on
+// the host).
 Status Solver::wait_status() {
+  const Status st = launched("solver step");
+  if (!st) return st;
   if (h_scalars_->flags & 8)
     return fail(HFPS_NUMERICAL_FAILURE, kDetailNumeric,
                 "small-level kernel: a grid barrier timed out");
@@ -2362,7 +2372,7 @@ Status Solver::apply_operator(const double* x, double* y, int memory) {
   if (!st) return st;
   if ((x + n <= y || y + n <= x) && in_place(y, n, memory)) out = y;
   launch_level_apply<double>(stream_, l64_[0].view(neumann_), in, out);
-  st = check(cudaGetLastError(), "operator launch");
+  st = launched("operator launch");
   if (st && out != y) st = copy_out(y, kap_, n, memory);
   if (!st) return st;
   return check(cudaStreamSynchronize(stream_), "operator");
@@ -2553,7 +2563,7 @@ Status Solver::profile_kernel(int kernel, int repetitions, double* ms,
   if (!st) return st;
   *ms = static_cast<double>(elapsed) / repetitions;
   *bytes = per_cell * cells;
-  return check(cudaGetLastError(), "profile kernels");
+  return launched("profile kernels");
 }
 
 }  // namespace hfps

@@ -87,6 +87,8 @@ class Solver {
   Status profile_kernel(int kernel, int repetitions, double* ms,
                         double* bytes);
   const std::string& last_error() const { return error_; }
+  // The calling thread's first refused launch since this was last asked.
+  Status launched(const char* what);
 
  private:
   Solver() = default;

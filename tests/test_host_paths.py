@@ -84,3 +84,31 @@ def test_shared_memory_limits_hold_for_every_handle(run, first, second, stretch)
     assert fake.fake_calls(b"cudaFuncSetAttribute") > 0
     assert fake.fake_lowered() == 0
     """)
+
+
+@pytest.mark.parametrize("call", ["apply", "update", "flux"])
+@pytest.mark.parametrize("shape,stretch", [((40, 40, 40), None), ((60, 24, 20), 0)])
+def test_refused_launch_is_reported(run, call, shape, stretch):
+    """Whichever launch of a call the runtime refuses, the call says so, no
+    graph that lacks the kernel is kept, and the next call is whole again."""
+    run(f"""
+    s = solver({shape}, {stretch})
+    c = [np.ones(n) for n in s.face_counts]
+    calls = {{"apply": lambda: apply(s), "update": lambda: update(s),
+              "flux": lambda: s.correct_flux(np.ones(s.cells), c, [v.copy() for v in c])}}
+    call = calls[{call!r}]
+    before = fake.fake_calls(b"cudaLaunchKernelExC")
+    call()
+    launches = fake.fake_calls(b"cudaLaunchKernelExC") - before
+    whole = fake.fake_launched(b"k_")
+    assert launches > 0 and (whole == launches or {call!r} != "apply")
+    for nth in range(1, launches + 1):
+        if {call!r} == "apply":
+            s = solver({shape}, {stretch})
+        graphs = fake.fake_calls(b"cudaGraphLaunch")
+        fake.fake_fail(b"cudaLaunchKernelExC", nth)
+        assert refused(call), nth
+        assert fake.fake_calls(b"cudaGraphLaunch") == graphs
+        call()
+        assert fake.fake_launched(b"k_") == whole
+    """)
