@@ -1254,12 +1254,13 @@ void Solver::mg_enqueue(std::vector<DeviceLevel<T>>& levels, const double* r,
   }
 }
 
+void Solver::clear_mg_graph(MgGraph& g) {
+  if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
+  if (g.graph != nullptr) cudaGraphDestroy(g.graph);
+  g = MgGraph{};
+}
 void Solver::clear_mg_graphs() {
-  for (MgGraph& g : mg_graph_) {
-    if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
-    if (g.graph != nullptr) cudaGraphDestroy(g.graph);
-    g = MgGraph{};
-  }
+  for (MgGraph& g : mg_graph_) clear_mg_graph(g);
 }
 
 // What a coefficient update can change in the kernels of an MG application.
@@ -1286,6 +1287,8 @@ cudaGraphNode_t Solver::captured_node() const {
 // update: 456x256x52, 31 of 163 ms.
 Status Solver::mg_retarget(MgGraph& g, const double* r, double* z) {
   if (g.r == r && g.z == z) return {};
+  g.r = nullptr;  // neither pair until every node is set
+  g.z = nullptr;
   // Argument positions of r and z (-1: none) in a kernel of `count` arguments.
   const auto set = [&](cudaGraphNode_t node, int count, int r_at, int z_at) -> Status {
     cudaKernelNodeParams params{};
@@ -1326,6 +1329,10 @@ Status Solver::mg_apply(bool mixed, const double* r, double* z) {
     return launched("mg launch");
   }
   MgGraph& g = mg_graph_[slot];
+  // Without its nodes a graph serves the pair it was captured for alone.
+  const bool nodes_known = g.enter != nullptr && g.exit != nullptr &&
+                           (policy_.unit_linear || g.projection != nullptr);
+  if (!nodes_known && (g.r != r || g.z != z)) clear_mg_graph(g);
   if (g.exec == nullptr) {
     MgGraph made;
     Status st = check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal),

@@ -264,6 +264,7 @@ class Solver {
   std::array<int, 8> mg_choices_{};
   std::array<int, 8> mg_choices() const;
   Status mg_retarget(MgGraph& g, const double* r, double* z);
+  static void clear_mg_graph(MgGraph& g);
   cudaGraphNode_t captured_node() const;
   size_t mg_nodes_[2]{};      // kernels per MG application (graph nodes)
   uint64_t launches_{};       // kernels launched since the last reset

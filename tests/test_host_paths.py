@@ -112,3 +112,36 @@ def test_refused_launch_is_reported(run, call, shape, stretch):
         call()
         assert fake.fake_launched(b"k_") == whole
     """)
+
+
+@pytest.mark.parametrize("unit", [1, 0])
+def test_graph_serves_the_vectors_of_its_call(run, unit):
+    """One captured application serves every pair of vectors: after an update
+    of its nodes that failed half-way, and where the capture could not tell
+    which nodes they are (then it is captured anew for another pair)."""
+    run(f"""
+    def pair(s):
+        return np.ones(s.cells), np.empty(s.cells)
+
+    def solve_on(s, v):
+        apply(s, v[0], z=v[1])
+        return fake.fake_entry_argument()
+
+    s = solver((20, 20, 20), unit_linear={unit})
+    first, second = pair(s), pair(s)
+    solve_on(s, first)
+    assert solve_on(s, second) == second[0].ctypes.data
+    for nth in range(1, 3 if {unit} else 4):
+        fake.fake_fail(b"cudaGraphExecKernelNodeSetParams", nth)
+        assert refused(lambda: solve_on(s, first)), nth
+        assert solve_on(s, second) == second[0].ctypes.data, nth
+    for nth in range(1, 3 if {unit} else 4):
+        s = solver((20, 20, 20), unit_linear={unit})
+        fake.fake_fail(b"cudaStreamGetCaptureInfo_v3", nth)
+        captures = fake.fake_calls(b"cudaStreamBeginCapture")
+        solve_on(s, first)
+        solve_on(s, first)
+        assert fake.fake_calls(b"cudaStreamBeginCapture") == captures + 1
+        solve_on(s, second)
+        assert fake.fake_calls(b"cudaStreamBeginCapture") == captures + 2, nth
+    """)
