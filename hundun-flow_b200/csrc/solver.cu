@@ -583,15 +583,16 @@ Status Solver::build_hierarchy() {
         return fail(HFPS_NUMERICAL_FAILURE, kDetailNumeric,
                     "non-positive coarse diagonal");
   }
-  coefficients_ready_ = true;
   mixed_ready_ = false;
   if (mg_choices() != mg_choices_) {
     clear_mg_graphs();
     mg_choices_ = mg_choices();
   }
   st = check(cudaStreamSynchronize(stream_), "hierarchy");
-  if (!st) return st;
-  return dic_factor();
+  if (st) st = launched("hierarchy kernels");
+  if (st) st = dic_factor();
+  coefficients_ready_ = bool(st);
+  return st;
 }
 
 // Cold-path IC(0) factorisation from the coefficients still staged in
@@ -608,10 +609,8 @@ Status Solver::dic_factor() {
   launch_dic_pivots(stream_, L0, dic_rows_, dic_inv_, dic_border_, d_scalars_);
   st = sync_scalars();
   if (!st) return st;
-  if (h_scalars_->flags & 1) {
-    coefficients_ready_ = false;
+  if (h_scalars_->flags & 1)
     return fail(HFPS_NUMERICAL_FAILURE, kDetailNumeric, "IC(0) pivot not positive");
-  }
   return {};
 }
 

@@ -145,3 +145,21 @@ def test_graph_serves_the_vectors_of_its_call(run, unit):
         solve_on(s, second)
         assert fake.fake_calls(b"cudaStreamBeginCapture") == captures + 2, nth
     """)
+
+
+def test_failed_factorisation_leaves_no_coefficients(run):
+    """An IC(0) factorisation that ends with any error (here a refused launch,
+    and the synchronisation that reads its status) leaves no pivots that a
+    later call could run on; the next update does."""
+    run("""
+    s = solver((20, 20, 20), preconditioner=hfps.solver.IC0)
+    for name in (b"cudaStreamSynchronize", b"cudaLaunchKernelExC"):
+        before = fake.fake_calls(name)
+        update(s)
+        calls = fake.fake_calls(name) - before  # the factorisation's are the last
+        fake.fake_fail(name, calls)
+        assert refused(lambda: update(s))
+        assert "coefficients not set" in refused(lambda: apply(s))
+        update(s)
+        apply(s)
+    """)
