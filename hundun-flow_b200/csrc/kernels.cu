@@ -1979,7 +1979,10 @@ void launch_chebyshev_stage(cudaStream_t s, const Level<T>& L, const T* x,
                             const T* b, T* direction, T* next,
                             T previous_factor, T residual_factor, bool first, bool last) {
   const long long cells = HFPS_CELLS(L);
-  if (cells >= kTiledStageCells) {
+  // The grid's second and third dimension hold 65535 tiles each; levels that
+  // long in y or z keep the flat kernel.
+  constexpr int kMaxTiles = 65535;
+  if (cells >= kTiledStageCells && L.ny <= kMaxTiles * kTileY && L.nz <= kMaxTiles * 8) {
     // Planes per tile as the tiled operator chooses them (tile_depth).
     int depth = 64;
     const long long columns = static_cast<long long>((L.nx + kTileX - 1) / kTileX) *

@@ -163,3 +163,15 @@ def test_failed_factorisation_leaves_no_coefficients(run):
         update(s)
         apply(s)
     """)
+
+
+@pytest.mark.parametrize("shape", [(2, 600000, 1), (1, 2, 600000), (600000, 2, 1)])
+@pytest.mark.parametrize("smoother", [0, 1])
+def test_long_grids_are_within_launch_limits(run, shape, smoother):
+    """Launch shapes of grids that are long in one direction: the second and
+    third grid dimension hold 65535 blocks each."""
+    run(f"""
+    s = solver({shape}, point_smoother={smoother})
+    for precision in (hfps.FP64, hfps.MIXED):
+        apply(s, precision=precision)
+    """)
