@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(ScanConfig<T>::threads)
 // the factors follow by asynchronous copies that hold no registers, each
 // thread then scans its chunk of up to ScanConfig<T>::rows rows out of shared
 // memory (chunks padded to an odd length, so that the lanes of a line fall in
-// different banks), and the solution goes back coalesced: 83 us, 2.6 TB/s of
+// different banks), and the solution goes back coalesced: 76 us, 2.8 TB/s of
 // the 36 bytes per cell that a pass needs (the transverse faces are 16 of them,
 // the factors 8).  A block of at most 2048 rows takes 52 KB of shared memory,
 // so that four blocks per SM overlap their load and scan phases; what bounds
@@ -413,7 +413,14 @@ struct ScanXShape {
   int pitch;        // shared-memory stride of a chunk
 };
 
-template <class T>
+// PARTS: a block has at most half as many lines as warps (long lines), and
+// several warps take a part each of a line in the load and store phases.  With a
+// warp per line whatever the block held, one warp of eight loaded 1030 FP32 rows
+// while the others waited (with the threads trimmed to the chunks, level-0 passes in
+// FP32: 700x140x140 206 -> 110 us, 1030x120x120 357 -> 128, 2048x90x90 372 -> 149;
+// FP64: 1030x120x120 370 -> 168, 2048x90x90 469 -> 189).  Shorter lines keep the
+// plain form, which the parts' bounds slow down (300x200x200 FP32 87 -> 105).
+template <class T, bool PARTS>
 __global__ void __launch_bounds__(kScanXThreads * (sizeof(T) == 4 ? 2 : 1))
     k_line_scan_x(Level<T> L, T* x, const T* __restrict__ rhs, const T* __restrict__ fac,
                   int color, ScanXShape sh) {
@@ -449,13 +456,19 @@ __global__ void __launch_bounds__(kScanXThreads * (sizeof(T) == 4 ? 2 : 1))
     fa = 2 * (t - fb * ha) + ((fb + color) & 1);
     return t < ha * L.nz && fa < L.ny;
   };
-  for (int l = warp; l < sh.lines; l += warps) {
+  // A warp's lines, and its rows of them.
+  const int share = PARTS ? max(1, warps / sh.lines) : 1;
+  const int first = PARTS ? warp / share : warp, next = PARTS ? warps / share : warps;
+  const int part = PARTS ? (extent + 32 * share - 1) / (32 * share) * 32 : 0;
+  const int row0 = PARTS ? (warp - first * share) * part + lane : lane;
+  const int row1 = PARTS ? min(extent, row0 - lane + part) : extent;
+  for (int l = first; l < sh.lines; l += next) {
     int fa, fb;
     if (!locate(t0 + l, fa, fb)) continue;
     const T* finv = fac + lay.cell(0, color, 0, t0 + l);
     const T* flow = fac + lay.cell(1, color, 0, t0 + l);
     const T* fup = fac + lay.cell(kSym ? 1 : 2, color, 0, t0 + l);
-    for (int s = lane; s < extent; s += 32) {
+    for (int s = row0; s < row1; s += 32) {
       const int at = l * line_pitch + place(s);
       copy_async(inv + at, finv + s);
       copy_async(up + at, fup + s);
@@ -463,7 +476,7 @@ __global__ void __launch_bounds__(kScanXThreads * (sizeof(T) == 4 ? 2 : 1))
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int l = warp; l < sh.lines; l += warps) {
+  for (int l = first; l < sh.lines; l += next) {
     int fa, fb;
     if (!locate(t0 + l, fa, fb)) continue;
     const LineRhs<T, 0, false> lr(L, fa, fb, 0);
@@ -472,7 +485,7 @@ __global__ void __launch_bounds__(kScanXThreads * (sizeof(T) == 4 ? 2 : 1))
     // FP64 their registers cost more than they give (13.0 -> 14.4 us a pass).
     constexpr int kInFlight = sizeof(T) == 4 ? 8 : 4;
 #pragma unroll kInFlight
-    for (int s = lane; s < extent; s += 32) {
+    for (int s = row0; s < row1; s += 32) {
       const int c = base + s;
       T v = __ldg(rhs + c);
 #pragma unroll
@@ -559,10 +572,10 @@ __global__ void __launch_bounds__(kScanXThreads * (sizeof(T) == 4 ? 2 : 1))
     }
   }
   __syncthreads();
-  for (int k = warp; k < sh.lines; k += warps) {
+  for (int k = first; k < sh.lines; k += next) {
     if (!locate(t0 + k, fa, fb)) continue;
     T* out = x + L.nx * (fa + L.ny * fb);
-    for (int s = lane; s < extent; s += 32) out[s] = d[k * line_pitch + place(s)];
+    for (int s = row0; s < row1; s += 32) out[s] = d[k * line_pitch + place(s)];
   }
 }
 
@@ -883,9 +896,18 @@ void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T*
   constexpr size_t arrays = 1 + ScanConfig<T>::arrays;
   const size_t smem =
       static_cast<size_t>(sh.lines) * sh.chunks * (arrays * sh.pitch + 4) * sizeof(T);
-  allow_shared(k_line_scan_x<T>, smem, threads * (arrays * (rows | 1) + 4) * sizeof(T));
-  launch(k_line_scan_x<T>, static_cast<int>((per_color + sh.lines - 1) / sh.lines), threads, smem,
-         s, L, x, b, fac, color, sh);
+  const size_t largest = threads * (arrays * (rows | 1) + 4) * sizeof(T);
+  // Threads for the chunks, and a warp per line to load with: 1030 FP32 rows are
+  // 129 chunks, and of a block of 256 threads half would only hold registers.
+  const int used =
+      std::min(threads, std::max((sh.lines * sh.chunks + 31) / 32 * 32, 32 * sh.lines));
+  const auto run = [&](auto kernel) {
+    allow_shared(kernel, smem, largest);
+    launch(kernel, static_cast<int>((per_color + sh.lines - 1) / sh.lines), used, smem, s, L, x, b,
+           fac, color, sh);
+  };
+  if (2 * 32 * sh.lines <= used) run(k_line_scan_x<T, true>);
+  else run(k_line_scan_x<T, false>);
 }
 
 template <class T, int AXIS>

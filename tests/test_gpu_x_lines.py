@@ -16,7 +16,9 @@ pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("oracle_built")]
 
 @pytest.mark.parametrize("shape,both", [
     ((33, 64, 40), False), ((100, 37, 61), False), ((257, 48, 48), False),
-    ((1030, 24, 46), False), ((71, 66, 63), True)])
+    ((1030, 24, 46), False), ((71, 66, 63), True),
+    # several warps per line: 2 to 8 of them, up to the longest line
+    ((520, 32, 33), False), ((700, 33, 32), False), ((2048, 32, 32), False)])
 def test_x_lines_match_restatement(cuda_library, shape, both):
     import c_oracle
     import hfps
