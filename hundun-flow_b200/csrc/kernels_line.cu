@@ -21,6 +21,7 @@
 #include "phase_device.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace hfps {
 namespace {
@@ -685,8 +686,14 @@ __global__ void __launch_bounds__(256)
 }
 
 // One zebra colour pass of the coarsest-level kernel for the lines handled
-// by this thread row (factors already in registers).
-template <class TC, int STEPS>
+// by this thread row (factors already in registers).  One CTA that solves a level
+// spends a pass on the latency of its factors and faces from L2, and exchanging
+// with two barriers a step is then the faster form (MG application with pcr_apply
+// instead: 60x60x40 1335 -> 1420 us, 257x48x48 2858 -> 2959, 31x72x72 2591 -> 2837;
+// with lines of 32 rows it gained, 32x72x72 2551 -> 2367); the CTAs that build the
+// dense map's columns hide that latency and take pcr_apply's (update of 200x40x40
+// 7.02 -> 6.74 ms).
+template <class TC, int STEPS, bool COLUMNS>
 __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
                                                  const TC* bs, TC* sd, int axis,
                                                  int fa, int fb, bool valid,
@@ -694,7 +701,25 @@ __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
                                                  const PcrRow<TC, STEPS>& r) {
   TC d = TC(0);
   if (valid && s < extent) d = line_rhs_any(L, xs, bs, axis, fa, fb, s, extent, c);
-  const TC value = pcr_apply(r, sd, s, d);
+  TC value;
+  if constexpr (COLUMNS) {
+    value = pcr_apply(r, sd, s, d);
+  } else {
+    constexpr int P = 1 << STEPS;
+    sd[s] = d;
+    __syncthreads();
+#pragma unroll
+    for (int step = 0; step < STEPS; ++step) {
+      const int lo = s - (1 << step), hi = s + (1 << step);
+      const TC dlo = lo >= 0 ? sd[lo] : TC(0);
+      const TC dhi = hi < P ? sd[hi] : TC(0);
+      const TC next = sd[s] - dlo * r.k[2 * step] - dhi * r.k[2 * step + 1];
+      __syncthreads();
+      sd[s] = next;
+      __syncthreads();
+    }
+    value = sd[s] / r.k[2 * STEPS];
+  }
   if (valid && s < extent) xs[c] = value;
   __syncthreads();
 }
@@ -703,12 +728,12 @@ __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
 // in shared memory (widened to TC).  When each colour's lines fit the CTA's
 // thread rows, both colours' PCR factors stay in registers for all sweeps.
 //
-// With kCoarseColumns, block j instead starts from unit data, x = e_j and
+// COLUMNS: with kCoarseColumns, block j instead starts from unit data, x = e_j and
 // b = 0 for j < n, x = 0 and b = e_{j-n} for j >= n, and writes its result
 // to x + j*n: the columns of the affine map x_out = P x_in + M b that the
 // sweeps apply (coarse_dense_operator).  kCoarseColumnsOn starts from the
 // column that is there, with the same b.
-template <class T, class TC, int STEPS>
+template <class T, class TC, int STEPS, bool COLUMNS>
 __global__ void __launch_bounds__(512)
     k_coarse_line_smem(Level<TC> L, T* __restrict__ x, const T* __restrict__ b,
                        const TC* __restrict__ fac, int sweeps, int axis,
@@ -722,7 +747,7 @@ __global__ void __launch_bounds__(512)
   TC* sd = bs + n + threadIdx.y * 2 * P;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   const int nthreads = blockDim.x * blockDim.y;
-  if (columns != kCoarseVector) {
+  if (COLUMNS) {
     const int j = blockIdx.x;
     x += static_cast<size_t>(j) * n;
     for (int c = tid; c < n; c += nthreads) {
@@ -767,8 +792,8 @@ __global__ void __launch_bounds__(512)
     pcr_load(fac, slab, at0, r0);
     pcr_load(fac, slab, at1, r1);
     for (int sweep = 0; sweep < sweeps; ++sweep) {
-      coarse_line_pass(L, xs, bs, sd, axis, fa0, fb0, v0, c0, s, extent, r0);
-      coarse_line_pass(L, xs, bs, sd, axis, fa1, fb1, v1, c1, s, extent, r1);
+      coarse_line_pass<TC, STEPS, COLUMNS>(L, xs, bs, sd, axis, fa0, fb0, v0, c0, s, extent, r0);
+      coarse_line_pass<TC, STEPS, COLUMNS>(L, xs, bs, sd, axis, fa1, fb1, v1, c1, s, extent, r1);
     }
   } else {
     for (int sweep = 0; sweep < sweeps; ++sweep) {
@@ -780,7 +805,7 @@ __global__ void __launch_bounds__(512)
           locate(base + threadIdx.y, color, fa, fb, valid, c, at);
           PcrRow<TC, STEPS> r;
           pcr_load(fac, slab, at, r);
-          coarse_line_pass(L, xs, bs, sd, axis, fa, fb, valid, c, s, extent, r);
+          coarse_line_pass<TC, STEPS, COLUMNS>(L, xs, bs, sd, axis, fa, fb, valid, c, s, extent, r);
         }
       }
     }
@@ -1062,15 +1087,17 @@ bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
   constexpr size_t kCoarseLineShared = 200 * 1024;
   if ((2 * cells + static_cast<size_t>(P) * lpb) * sizeof(TC) > kCoarseLineShared) return false;
   const size_t smem = (2 * cells + static_cast<size_t>(2) * P * lpb) * sizeof(TC);
-  const dim3 block(P, lpb);
+  const auto run = [&](auto kernel, int blocks) {
+    allow_shared(kernel, smem, kCoarseLineShared + 512 * sizeof(TC));
+    launch(kernel, blocks, dim3(P, lpb), smem, s, L, x, b, fac, sweeps, axis, columns);
+  };
   switch (steps) {
 #define HFPS_COARSE_CASE(N)                                                      \
   case N:                                                                        \
-    allow_shared(k_coarse_line_smem<T, TC, N>, smem,                             \
-                 kCoarseLineShared + 512 * sizeof(TC));                          \
-    launch(k_coarse_line_smem<T, TC, N>,                                          \
-           columns != kCoarseVector ? 2 * static_cast<int>(cells) : 1, block, smem, s, L, x, \
-           b, fac, sweeps, axis, columns);                                         \
+    if (columns == kCoarseVector) run(k_coarse_line_smem<T, TC, N, false>, 1);    \
+    else if constexpr (std::is_same<T, TC>::value)                                \
+      run(k_coarse_line_smem<T, TC, N, true>, 2 * static_cast<int>(cells));       \
+    else return false;                                                            \
     break;
     HFPS_COARSE_CASE(0) HFPS_COARSE_CASE(1) HFPS_COARSE_CASE(2) HFPS_COARSE_CASE(3)
     HFPS_COARSE_CASE(4) HFPS_COARSE_CASE(5) HFPS_COARSE_CASE(6) HFPS_COARSE_CASE(7)

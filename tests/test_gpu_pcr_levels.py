@@ -52,3 +52,29 @@ def test_pcr_levels_match_restatement(cuda_library, axis, rows, others, pre, pos
     assert np.linalg.norm(g.apply_preconditioner(r) - expected) <= 1e-11 * size
     mixed = g.apply_preconditioner(r, precision=hfps.MIXED)
     assert np.linalg.norm(mixed - expected) <= max(shape) ** 2 * 2.0 ** -24 * size
+
+
+@pytest.mark.parametrize("axis,rows,others,extent", [
+    (0, 16, (26, 26), 13), (0, 31, (18, 18), 9), (1, 32, (18, 18), 9), (2, 60, (18, 18), 9),
+    (1, 100, (10, 10), 5), (0, 130, (10, 10), 5)])
+def test_coarsest_line_levels_match_restatement(cuda_library, axis, rows, others, extent):
+    """Coarsest levels of more cells than the dense map holds are swept by one
+    CTA: rows of 16 (exchanged as longer ones are) to 130."""
+    import c_oracle
+    import hfps
+    import ref_oracle
+    shape = list(others)
+    shape.insert(axis, rows)
+    s = stretched_front(tuple(shape), axis, 1.0 + 3.0 / rows)
+    policy = hfps.Policy.production().replace(anisotropy_threshold=4.0,
+                                              minimum_coarse_extent=extent)
+    g = hfps.PressureSolver.from_system(s, policy)
+    assert g.levels()[0][3] == 1 << axis
+    assert np.prod(g.levels()[-1][:3]) > 2048
+    oracle = c_oracle.OracleSession(
+        s, ref_oracle.MgPolicy(smoother=1, cycle=1, pre=1, post=2, diagonal_shortcut=0.1,
+                               min_coarse_extent=extent, anisotropy_threshold=4.0),
+        unit_linear=True, line_order=1)
+    r = np.ascontiguousarray(workloads.normals(3, s.cells).reshape(s.rhs.shape))
+    expected = oracle.apply_mg(r)
+    assert np.linalg.norm(g.apply_preconditioner(r) - expected) <= 1e-11 * np.linalg.norm(expected)
