@@ -502,6 +502,7 @@ void Solver::aggregate_channel(int level, int face_axis, const double* src,
 }
 
 Status Solver::build_hierarchy() {
+  coefficients_ready_ = false;  // until the whole update has succeeded
   for (size_t l = 1; l < l64_.size(); ++l) {
     const DeviceLevel<double>& F = l64_[l - 1];
     DeviceLevel<double>& C = l64_[l];

@@ -147,21 +147,23 @@ def test_graph_serves_the_vectors_of_its_call(run, unit):
     """)
 
 
-def test_failed_factorisation_leaves_no_coefficients(run):
-    """An IC(0) factorisation that ends with any error (here a refused launch,
-    and the synchronisation that reads its status) leaves no pivots that a
-    later call could run on; the next update does."""
-    run("""
-    s = solver((20, 20, 20), preconditioner=hfps.solver.IC0)
+@pytest.mark.parametrize("preconditioner,stretch", [("IC0", None), ("MG", None), ("MG", 1)])
+def test_failed_update_leaves_no_coefficients(run, preconditioner, stretch):
+    """An update that ends with any error (a refused launch, or one of the
+    synchronisations that read what it found; the IC(0) factorisation's are the
+    last) leaves no levels or pivots that a later call could run on; the next
+    update does."""
+    run(f"""
+    s = solver((20, 30, 20), {stretch}, preconditioner=hfps.solver.{preconditioner})
     for name in (b"cudaStreamSynchronize", b"cudaLaunchKernelExC"):
         before = fake.fake_calls(name)
         update(s)
-        calls = fake.fake_calls(name) - before  # the factorisation's are the last
-        fake.fake_fail(name, calls)
-        assert refused(lambda: update(s))
-        assert "coefficients not set" in refused(lambda: apply(s))
-        update(s)
-        apply(s)
+        for nth in range(1, fake.fake_calls(name) - before + 1):
+            fake.fake_fail(name, nth)
+            assert refused(lambda: update(s))
+            assert "coefficients not set" in refused(lambda: apply(s)), (name, nth)
+            update(s)
+            apply(s)
     """)
 
 
