@@ -537,17 +537,16 @@ Status Solver::build_hierarchy() {
   if (!st) return st;
   select_tail();
   select_small();
-  line_ends_ = true;
-  if (l64_[0].line_mask != 0) {
+  // Read after the synchronisation that ends the update.
+  const bool lines = l64_[0].line_mask != 0;
+  if (lines) {
     st = check(cudaMemsetAsync(&d_scalars_->marks, 0, sizeof(unsigned), stream_), "boundary faces");
     if (!st) return st;
     launch_neumann_faces(stream_, l64_[0].view(neumann_), d_scalars_);
     st = check(cudaMemcpyAsync(&h_scalars_->marks, &d_scalars_->marks, sizeof(unsigned),
                                cudaMemcpyDeviceToHost, stream_),
                "boundary faces");
-    if (st) st = check(cudaStreamSynchronize(stream_), "boundary faces");
     if (!st) return st;
-    line_ends_ = (h_scalars_->marks & 2u) != 0;
   }
   // Diagonal shortcut (select_diagonal_shortcut, src/solver_mg.cpp:1577-1611).
   diagonal_shortcut_ = false;
@@ -585,12 +584,13 @@ Status Solver::build_hierarchy() {
                     "non-positive coarse diagonal");
   }
   mixed_ready_ = false;
+  st = check(cudaStreamSynchronize(stream_), "hierarchy");
+  if (st) st = launched("hierarchy kernels");
+  line_ends_ = !(st && lines) || (h_scalars_->marks & 2u) != 0;
   if (mg_choices() != mg_choices_) {
     clear_mg_graphs();
     mg_choices_ = mg_choices();
   }
-  st = check(cudaStreamSynchronize(stream_), "hierarchy");
-  if (st) st = launched("hierarchy kernels");
   if (st) st = dic_factor();
   coefficients_ready_ = bool(st);
   return st;
