@@ -22,24 +22,22 @@
 // kernel therefore starts with grid_dependency_sync(), which waits until the
 // preceding grid has completed and its writes are visible, before touching
 // any memory.  Kernels launched without the attribute pass it straight
-// through.  An early launch_dependents trigger (dependents scheduled while
-// this grid still runs) measured slower at 256^3: 7% on the FP32 MG cycle,
-// and 3% on the FP64 one when given to the FP64 kernels alone (2.79 -> 2.88
-// ms), so dependents launch at grid exit.
+// through.  Two kernels read ahead of the wait: k_small_cycle its levels'
+// coefficients and k_line_pcr_sweeps its first pass's factors, neither of which
+// the preceding grid writes.  That is safe only because no kernel triggers its
+// dependents early: a grid that starts before its predecessor has ended still
+// starts after the predecessor's own wait, so every grid before that one, the
+// writers of the coefficients and factors among them, has completed.  An early
+// trigger also measured slower at 256^3: 7% on the FP32 MG cycle, and 3% on the
+// FP64 one when given to the FP64 kernels alone (2.79 -> 2.88 ms).
 #ifndef HFPS_USE_PDL
 #define HFPS_USE_PDL 1
-#endif
-#ifndef HFPS_PDL_EARLY_TRIGGER
-#define HFPS_PDL_EARLY_TRIGGER 0
 #endif
 
 namespace hfps {
 
 __device__ __forceinline__ void grid_dependency_sync() {
 #if HFPS_USE_PDL
-#if HFPS_PDL_EARLY_TRIGGER
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
   asm volatile("griddepcontrol.wait;" ::: "memory");
 #endif
 }
