@@ -114,10 +114,9 @@ struct LineRhs {
   }
 
   // Row s, c its vector index.  MODE kScanFresh: x is zero everywhere, so the
-  // row is the rhs alone (every term is a finite face times zero).
-  // ENDS: a Neumann
-  // face at a line end may be nonzero; otherwise the end terms are exact zeros
-  // and the cell's own x is not read.
+  // row is the rhs alone (every term is a finite face times zero).  ENDS: a
+  // Neumann face at a line end may be nonzero; otherwise the end terms are exact
+  // zeros and the cell's own x is not read.
   template <int MODE, bool ENDS>
   __device__ __forceinline__ T row(const T* x, const T* __restrict__ rhs, int c,
                                    int s, int extent) const {
@@ -860,8 +859,8 @@ ScanShape scan_shape(long long per_color, int extent) {
 // and levels that three blocks per SM hold anyway gain nothing (64x256x64 9.9 ->
 // 11.0 us, 32x256x32 7.3 -> 8.3): those keep the kernel with the end terms,
 // which are exact zeros then.  FP32 has 64 registers and two blocks per SM either
-// way, and its level-0 pass is slower without them (94.5 -> 100.3 us), but for the
-// fresh one, which then reads nothing but rhs.
+// way, and its level-0 pass is slower without them (94.5 -> 100.3 us).  A fresh pass
+// reads nothing but rhs in either form.
 struct ScanFlags {
   int hx;
   bool zero_other, zero_self, ends;
@@ -873,34 +872,28 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
   const int blocks = static_cast<int>((per_color + LPB - 1) / LPB);
   const size_t smem = static_cast<size_t>(4) * sh.chunks * LPB * sizeof(T);
   const dim3 block(LPB, sh.chunks);
-  // Without end terms the zero flag is an argument of the ordinary kernel (a
-  // kernel of its own takes more registers); with them it is a mode.
-  const bool fresh = f.zero_other && f.zero_self;
-  const bool ends = f.ends || f.hx == 0 || blocks <= 3 * 148 || (sizeof(T) == 4 && !fresh);
-  const int mode = fresh ? kScanFresh : (f.zero_self && ends ? kScanOwnZero : kScanNormal);
   const bool split = f.hx != 0;
-#define HFPS_SCAN_RUN(MODE, SPLIT, ENDS)                                                    \
-  launch(k_line_scan_color<T, AXIS, LPB, MODE, SPLIT, ENDS>, blocks, block, smem, s, L, x, b, \
-         fac, color, sh.rows, f.hx, f.zero_self)
-#define HFPS_SCAN_ENDS(MODE, SPLIT) HFPS_SCAN_RUN(MODE, SPLIT, true)
-#define HFPS_SCAN_LAUNCH(MODE, SPLIT)                                                       \
-  do {                                                                                      \
-    if (ends) HFPS_SCAN_RUN(MODE, SPLIT, true);                                             \
-    else HFPS_SCAN_RUN(MODE, SPLIT, false);                                                 \
-  } while (0)
-  if (mode == kScanFresh) {
-    if (split) HFPS_SCAN_LAUNCH(kScanFresh, true);
-    else HFPS_SCAN_LAUNCH(kScanFresh, false);
-  } else if (mode == kScanOwnZero) {
-    if (split) HFPS_SCAN_ENDS(kScanOwnZero, true);
-    else HFPS_SCAN_ENDS(kScanOwnZero, false);
-  } else {
-    if (split) HFPS_SCAN_LAUNCH(kScanNormal, true);
-    else HFPS_SCAN_LAUNCH(kScanNormal, false);
+  const auto run = [&](auto kernel) {
+    launch(kernel, blocks, block, smem, s, L, x, b, fac, color, sh.rows, f.hx, f.zero_self);
+  };
+  // The kernel without end terms takes the zero flag as an argument (a kernel of
+  // its own takes more registers); with them it is a mode.
+  if constexpr (sizeof(T) == 8) {
+    if (!f.ends && split && blocks > 3 * 148 && !(f.zero_other && f.zero_self)) {
+      run(k_line_scan_color<T, AXIS, LPB, kScanNormal, true, false>);
+      return;
+    }
   }
-#undef HFPS_SCAN_LAUNCH
-#undef HFPS_SCAN_ENDS
-#undef HFPS_SCAN_RUN
+  if (f.zero_other && f.zero_self) {
+    if (split) run(k_line_scan_color<T, AXIS, LPB, kScanFresh, true, true>);
+    else run(k_line_scan_color<T, AXIS, LPB, kScanFresh, false, true>);
+  } else if (f.zero_self) {
+    if (split) run(k_line_scan_color<T, AXIS, LPB, kScanOwnZero, true, true>);
+    else run(k_line_scan_color<T, AXIS, LPB, kScanOwnZero, false, true>);
+  } else {
+    if (split) run(k_line_scan_color<T, AXIS, LPB, kScanNormal, true, true>);
+    else run(k_line_scan_color<T, AXIS, LPB, kScanNormal, false, true>);
+  }
 }
 
 // As many lines per block as its threads have chunks for, halved (down to one
