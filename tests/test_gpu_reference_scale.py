@@ -92,6 +92,9 @@ def test_live_reference_full_vectors(hfps_mod):
     """256^3 and 128^3, PCG and FGMRES(12), cold and warm: the compiled
     reference runs in spawned processes (one per solve) while the GPU
     solves the same systems."""
+    import ref_oracle
+    if not ref_oracle.available():
+        pytest.skip("compiled reference not built (make -C oracle ref)")
     import torch
     cases = [(name, a) for name in ("wrinkled256", "wrinkled128") for a in ("pcg", "fgmres")]
     with tempfile.TemporaryDirectory() as tmp, scale_cases.reference_pool(8) as pool:

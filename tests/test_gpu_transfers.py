@@ -55,3 +55,22 @@ def test_prolongation_with_first_step_matches_restatement(cuda_library, shape, p
     z = hfps.PressureSolver.from_system(s, policy).apply_preconditioner(r)
     oracle = c_oracle.OracleSession(s, mg, unit_linear=True)
     assert np.array_equal(z, oracle.apply_mg(r))
+
+
+@pytest.mark.parametrize("shape", [(103, 101, 107), (40, 163, 165)])
+@pytest.mark.parametrize("pre,post", [(3, 1), (1, 3)])
+def test_tiled_stages_match_restatement(cuda_library, shape, pre, post):
+    """Chebyshev stages over 3-D tiles, levels of at least 2^20 cells: tiles cut
+    in every direction, and the first, middle and last stage and the only one."""
+    import c_oracle
+    import hfps
+    import ref_oracle
+    s = workloads.make("sphere64", n=shape, seed=6)
+    assert s.cells >= 1 << 20
+    policy = hfps.Policy.production().replace(pre_sweeps=pre, post_sweeps=post,
+                                              anisotropy_threshold=1e3)
+    mg = ref_oracle.MgPolicy(smoother=1, cycle=1, pre=pre, post=post, diagonal_shortcut=0.1,
+                             anisotropy_threshold=1e3)
+    r = np.ascontiguousarray(workloads.normals(3, s.cells).reshape(s.rhs.shape))
+    z = hfps.PressureSolver.from_system(s, policy).apply_preconditioner(r)
+    assert np.array_equal(z, c_oracle.OracleSession(s, mg, unit_linear=True).apply_mg(r))
