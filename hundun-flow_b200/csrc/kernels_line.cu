@@ -686,13 +686,14 @@ __global__ void __launch_bounds__(256)
 
 // One zebra colour pass of the coarsest-level kernel for the lines handled
 // by this thread row (factors already in registers).  One CTA that solves a level
-// spends a pass on the latency of its factors and faces from L2, and exchanging
-// with two barriers a step is then the faster form (MG application with pcr_apply
-// instead: 60x60x40 1335 -> 1420 us, 257x48x48 2858 -> 2959, 31x72x72 2591 -> 2837;
-// with lines of 32 rows it gained, 32x72x72 2551 -> 2367); the CTAs that build the
-// dense map's columns hide that latency and take pcr_apply's (update of 200x40x40
-// 7.02 -> 6.74 ms).
-template <class TC, int STEPS, bool COLUMNS>
+// spends a pass on the latency of its factors and faces from L2, and which exchange
+// is faster depends on the rows: pcr_apply's where they fill the threads of a line
+// (ONE_BARRIER; MG application with two barriers a step, then with one: 32x72x72 2551
+// and 2367 us, 256x48x48 1544 and 1498), two barriers a step where some threads hold
+// no row (31x72x72 2591 and 2837, 60x60x40 1335 and 1420, 240x40x40 1557 and 1570,
+// 257x48x48 2858 and 2959).  The CTAs that build the dense map's columns hide the
+// latency and take pcr_apply's (update of 200x40x40 7.02 -> 6.74 ms).
+template <class TC, int STEPS, bool ONE_BARRIER>
 __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
                                                  const TC* bs, TC* sd, int axis,
                                                  int fa, int fb, bool valid,
@@ -701,7 +702,7 @@ __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
   TC d = TC(0);
   if (valid && s < extent) d = line_rhs_any(L, xs, bs, axis, fa, fb, s, extent, c);
   TC value;
-  if constexpr (COLUMNS) {
+  if constexpr (ONE_BARRIER) {
     value = pcr_apply(r, sd, s, d);
   } else {
     constexpr int P = 1 << STEPS;
@@ -732,7 +733,7 @@ __device__ __forceinline__ void coarse_line_pass(const Level<TC>& L, TC* xs,
 // to x + j*n: the columns of the affine map x_out = P x_in + M b that the
 // sweeps apply (coarse_dense_operator).  kCoarseColumnsOn starts from the
 // column that is there, with the same b.
-template <class T, class TC, int STEPS, bool COLUMNS>
+template <class T, class TC, int STEPS, bool COLUMNS, bool ONE_BARRIER>
 __global__ void __launch_bounds__(512)
     k_coarse_line_smem(Level<TC> L, T* __restrict__ x, const T* __restrict__ b,
                        const TC* __restrict__ fac, int sweeps, int axis,
@@ -791,8 +792,10 @@ __global__ void __launch_bounds__(512)
     pcr_load(fac, slab, at0, r0);
     pcr_load(fac, slab, at1, r1);
     for (int sweep = 0; sweep < sweeps; ++sweep) {
-      coarse_line_pass<TC, STEPS, COLUMNS>(L, xs, bs, sd, axis, fa0, fb0, v0, c0, s, extent, r0);
-      coarse_line_pass<TC, STEPS, COLUMNS>(L, xs, bs, sd, axis, fa1, fb1, v1, c1, s, extent, r1);
+      coarse_line_pass<TC, STEPS, ONE_BARRIER>(L, xs, bs, sd, axis, fa0, fb0, v0, c0, s, extent,
+                                               r0);
+      coarse_line_pass<TC, STEPS, ONE_BARRIER>(L, xs, bs, sd, axis, fa1, fb1, v1, c1, s, extent,
+                                               r1);
     }
   } else {
     for (int sweep = 0; sweep < sweeps; ++sweep) {
@@ -804,7 +807,8 @@ __global__ void __launch_bounds__(512)
           locate(base + threadIdx.y, color, fa, fb, valid, c, at);
           PcrRow<TC, STEPS> r;
           pcr_load(fac, slab, at, r);
-          coarse_line_pass<TC, STEPS, COLUMNS>(L, xs, bs, sd, axis, fa, fb, valid, c, s, extent, r);
+          coarse_line_pass<TC, STEPS, ONE_BARRIER>(L, xs, bs, sd, axis, fa, fb, valid, c, s,
+                                                   extent, r);
         }
       }
     }
@@ -1087,9 +1091,12 @@ bool launch_coarse_line(cudaStream_t s, const Level<TC>& L, T* x, const T* b,
   switch (steps) {
 #define HFPS_COARSE_CASE(N)                                                      \
   case N:                                                                        \
-    if (columns == kCoarseVector) run(k_coarse_line_smem<T, TC, N, false>, 1);    \
+    if (columns == kCoarseVector && extent == 1 << N)                             \
+      run(k_coarse_line_smem<T, TC, N, false, true>, 1);                          \
+    else if (columns == kCoarseVector)                                            \
+      run(k_coarse_line_smem<T, TC, N, false, false>, 1);                         \
     else if constexpr (std::is_same<T, TC>::value)                                \
-      run(k_coarse_line_smem<T, TC, N, true>, 2 * static_cast<int>(cells));       \
+      run(k_coarse_line_smem<T, TC, N, true, true>, 2 * static_cast<int>(cells)); \
     else return false;                                                            \
     break;
     HFPS_COARSE_CASE(0) HFPS_COARSE_CASE(1) HFPS_COARSE_CASE(2) HFPS_COARSE_CASE(3)

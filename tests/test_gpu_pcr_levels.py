@@ -58,10 +58,10 @@ def test_pcr_levels_match_restatement(cuda_library, axis, rows, others, pre, pos
 
 @pytest.mark.parametrize("axis,rows,others,extent", [
     (0, 16, (26, 26), 13), (0, 31, (18, 18), 9), (1, 32, (18, 18), 9), (2, 60, (18, 18), 9),
-    (1, 100, (10, 10), 5), (0, 130, (10, 10), 5)])
+    (2, 64, (18, 18), 9), (1, 100, (10, 10), 5), (0, 130, (10, 10), 5), (0, 256, (10, 10), 5)])
 def test_coarsest_line_levels_match_restatement(cuda_library, axis, rows, others, extent):
     """Coarsest levels of more cells than the dense map holds are swept by one
-    CTA: rows of 16 (exchanged as longer ones are) to 130."""
+    CTA: rows that fill the threads of a line, and rows that do not."""
     import c_oracle
     import hfps
     import ref_oracle
