@@ -352,10 +352,10 @@ def run_reference(args, world, rank):
 
 
 # DRAM bytes per level-0 cell of one zebra colour pass of the FP64 line
-# kernel (split-row vectors, a pass that reads x), from one ncu capture at
-# 256x256x128 (337.1 MB read + 26.1 MB written over 8,388,608 cells);
-# traffic grows with the cell count.
-LINE_PASS_DRAM_BYTES_PER_CELL = (303.605760e6 + 26.895872e6) / (256 * 256 * 128)
+# kernel (split-row vectors, no end terms, a pass that reads x), from one ncu
+# capture at 256x256x128 (274.5 MB read + 22.5 MB written over 8,388,608
+# cells); traffic grows with the cell count.
+LINE_PASS_DRAM_BYTES_PER_CELL = (274.468096e6 + 22.533120e6) / (256 * 256 * 128)
 
 def reference_solution_errors(args, solver, rhs0):
     """Relative L2 error, over the recorded sample of cells, of the FP64 and
@@ -515,7 +515,7 @@ def run_b200(args, world, rank, local):
         peak, peak_note = 6650.0, "fallback"
     dom = kernels["smooth_fp64"]
     roofline = {"bound": "hbm",
-                "kernel": "k_line_scan_color<double,y,8,normal,split rows> level 0 "
+                "kernel": "k_line_scan_color<double,y,8,normal,split rows,no end terms> level 0 "
                           "(one zebra colour)",
                 "achieved": dom["gbs"], "peak": peak, "unit": "GB/s",
                 "frac": dom["gbs"] / peak, "peak_source": peak_note,
