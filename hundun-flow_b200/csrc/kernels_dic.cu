@@ -18,16 +18,19 @@
 // tile waits for the entries themselves.  No flag, fence or barrier lies between
 // two tiles (a flag per 8 steps cost 3.4 us each in its wait, loads and fence).
 //
-// What bounds it: the chain of nx + ny + nz dependent steps and one way through
-// L2 per tile border.  A step is some twenty instructions of one warp per
-// scheduler, so nothing else may run in the compute warps: four more warps copy
-// the next chunk's inputs to shared memory (cp.async, the skewed windows of all
-// rows, kDicChunk steps), wait for its border entries and write the last chunk's
-// results back.  With all of it in the four compute warps a step took 0.36 us,
-// now 0.18 forward and 0.25 backward.  Steps outside the grid compute on whatever
+// What bounds it: the chain of nx + ny + nz - 2 dependent steps, and 2.2 us per
+// tile border on the longest path beyond the steps of its skew: the copy warps wait
+// for all border entries of a chunk before the barrier that starts it, up to seven
+// steps more than the skew needs, and the entries take a trip through L2.  A step is
+// some twenty instructions of one warp per scheduler, so nothing else may run in
+// the compute warps: four more warps copy the next chunk's inputs to shared memory
+// (cp.async, the skewed windows of all rows, kDicChunk steps), wait for its border
+// entries and write the last chunk's results back.  With all of it in the four
+// compute warps a step took 0.36 us, now 0.18 forward and 0.25 backward.  Steps outside the grid compute on whatever
 // is there and are set to zero, which is also the neighbour outside it, so a step
-// has no branches.  The sweeps of an application take 72 + 83 us at 64^3 and
-// 236 + 257 at 128^3.
+// has no branches.  The sweeps of an application take 72 + 83 us at 64^3, where the
+// longest path has 190 steps (34 + 47 us) and ten borders (22 us a sweep; some 15 us
+// a sweep are neither), and 236 + 257 at 128^3.
 //
 // Waits cannot deadlock: tiles are taken in the order of a ticket, diagonal by
 // diagonal, so a tile waits only for tiles whose CTAs are already running.

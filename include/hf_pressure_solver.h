@@ -219,7 +219,9 @@ HFPS_API int hfps_create(const hfps_geometry* geometry, const hfps_policy* polic
  * (src/solver_ibm_pressure.cpp:347-385) and copy_finest_coefficients
  * (src/solver_mg.cpp:1469-1570) do; then the coarse levels are aggregated
  * (build_coarse_coefficients, src/solver_mg.cpp:1858-1925).  Replaces
- * NativeCartesianMgPlan::update_coefficients (v04_linear.hpp:955-960). */
+ * NativeCartesianMgPlan::update_coefficients (v04_linear.hpp:955-960).
+ * After this, hfps_set_beta or hfps_assemble failed while it built the levels,
+ * calls that need coefficients return HFPS_INVALID_PLAN until one succeeds. */
 HFPS_API int hfps_set_coefficients(hfps_solver* solver, const double* diagonal,
                           const double* face_x, const double* face_y,
                           const double* face_z, int memory);
