@@ -305,15 +305,18 @@ __device__ void line_thomas(const Level<T>& L, T* x, const T* b, T* work,
   }
 }
 
-// x (and the first Chebyshev direction) of cell c, whose rhs is `b`, by `zero`.
-// START is whether its kind is a smoothing step, fixed at compile time: as a
+// x (and the first Chebyshev direction) of coarse cell c, whose rhs is `b`, by
+// `zero`.  START is whether its kind is a smoothing step, fixed at compile time: as a
 // run-time choice it slowed the line levels' restriction and entry (MG
-// application at 256^3 2.917 -> 2.956 ms, with it 2.929).
+// application at 256^3 2.917 -> 2.956 ms, with it 2.929).  Without one x is cleared,
+// also where nothing reads it (kZeroNone, the one-CTA levels): a look at the kind
+// took the FP64 restriction over x and y from 32 to 36 registers (90x73x299 23.2 ->
+// 27.3 us).
 template <bool START, class T>
 __device__ __forceinline__ void write_zero_start(const ZeroStart<T>& zero, T b, T* x, int c,
                                                  int parity) {
   if (!START) {
-    if (zero.kind != kZeroNone) x[c] = T(0);
+    x[c] = T(0);
     return;
   }
   T d;
