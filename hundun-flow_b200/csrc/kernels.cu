@@ -2144,10 +2144,13 @@ long long tile_count(const Level<double>& L, int depth) {
   return static_cast<long long>((L.nx + kTileX - 1) / kTileX) *
          ((L.ny + kTileY - 1) / kTileY) * ((L.nz + depth - 1) / depth);
 }
-// Planes per tile: the deepest of 64, 32, 16, 8, 4, 2 that still gives at least
-// three quarters of a wave of resident tiles (8 per SM), so that mid-size
-// grids run in about one full wave and small ones are not left to a few SMs
-// (64^3: 8 planes, 128 tiles 10.2 us; 2 planes, 512 tiles 7.4).
+// Planes per tile: the deepest of 64, 32, 16, 8 that still gives at least three
+// quarters of a wave of resident tiles (8 per SM), so that mid-size grids run in
+// about one full wave.  Small grids are not left to a few SMs: 2 planes, or else
+// 4, where that gives at most 5 tiles per SM (64^3: 8 planes, 128 tiles 9.1 us; 4
+// planes 6.9; 2 planes, 512 tiles 6.6.  72^3: 8 planes 9.9 us, 4 planes, 486 tiles
+// 8.5, 2 planes, 972 tiles 9.1).  With more, a shallow tile's extra two planes of x
+// cost what the tiles give (104^3: 8 planes 14.5 us, 4 planes, 1352 tiles 16.6).
 int tile_depth(const Level<double>& L) {
   static const int wave = [] {
     int device = 0, sms = 0;
@@ -2155,8 +2158,10 @@ int tile_depth(const Level<double>& L) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     return 8 * (sms > 0 ? sms : 148);
   }();
+  for (int shallow = 2; shallow < 8; shallow *= 2)
+    if (8 * tile_count(L, shallow) <= 5LL * wave) return shallow;
   int depth = 64;
-  while (depth > 2 && 4 * tile_count(L, depth) < 3LL * wave) depth >>= 1;
+  while (depth > 8 && 4 * tile_count(L, depth) < 3LL * wave) depth >>= 1;
   return depth;
 }
 
