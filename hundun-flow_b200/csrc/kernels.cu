@@ -1096,14 +1096,16 @@ __global__ void __launch_bounds__(kTileX * kTileY)
     apply_scalar_op(red.scalars, red.op, acc[0]);
 }
 
-// One Chebyshev stage of a large level over the same tiles: the flat kernel
+// One FP32 Chebyshev stage of a large level over the same tiles: the flat kernel
 // (k_chebyshev_stage) reads x three times and the faces twice through L2, which
-// bounds it there; here each plane comes once.  At 512x256x256 FP32 a pair of
-// stages went from 524 us to 448 (32 and 32 bytes per cell: 161 us each; some of
-// it is the last direction that is no longer stored), at 128^3 from 31.5 to 28.9;
-// below kTiledStageCells the tiles march too few planes each (64^3 FP64 8.4 ->
-// 14.6).
-constexpr long long kTiledStageCells = 1LL << 20;
+// bounds it there; here each plane comes once, for more instructions a cell.  It
+// gains while few of a wave's places are empty: with 8 tiles per SM and each tile
+// its full cells, at least kTiledStageFill of them must be the level's (FP32 stage,
+// flat and tiled: 512x256x256 279 and 241 us, 256^3 137 and 124, 128^3 16.8 and
+// 15.1, 153x325x151 62.5 and 60.2, all above; below, 288^3 196 and 214, 176^3 47
+// and 53, 161x160x160 37 and 48, 48x400x400 65 and 93).  FP64, whose flat kernel
+// is at the same bytes' bound, gains nothing (256^3 214 and 216, 250^3 202 and 213).
+constexpr double kTiledStageFill = 0.75;
 
 template <class T, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kTileX * kTileY)
@@ -1982,27 +1984,30 @@ void launch_chebyshev_stage(cudaStream_t s, const Level<T>& L, const T* x,
                             const T* b, T* direction, T* next,
                             T previous_factor, T residual_factor, bool first, bool last) {
   const long long cells = HFPS_CELLS(L);
-  // The grid's second and third dimension hold 65535 tiles each; levels that
-  // long in y or z keep the flat kernel.
-  constexpr int kMaxTiles = 65535;
-  if (cells >= kTiledStageCells && L.ny <= kMaxTiles * kTileY && L.nz <= kMaxTiles * 8) {
+  if constexpr (sizeof(T) == 4) {
     // Planes per tile as the tiled operator chooses them (tile_depth).
-    int depth = 64;
     const long long columns = static_cast<long long>((L.nx + kTileX - 1) / kTileX) *
                               ((L.ny + kTileY - 1) / kTileY);
-    while (depth > 8 && 4 * columns * ((L.nz + depth - 1) / depth) < 3 * 148LL * 8) depth >>= 1;
+    constexpr long long wave = 148LL * 8;
+    int depth = 64;
+    while (depth > 8 && 4 * columns * ((L.nz + depth - 1) / depth) < 3 * wave) depth >>= 1;
     const dim3 grid((L.nx + kTileX - 1) / kTileX, (L.ny + kTileY - 1) / kTileY,
                     (L.nz + depth - 1) / depth);
-    const dim3 block(kTileX, kTileY);
-    const auto run = [&](auto kernel) {
-      launch(kernel, grid, block, 0, s, L, x, b, direction, next, previous_factor,
-             residual_factor, depth);
-    };
-    if (first && last) run(k_chebyshev_tiled<T, true, true>);
-    else if (first) run(k_chebyshev_tiled<T, true, false>);
-    else if (last) run(k_chebyshev_tiled<T, false, true>);
-    else run(k_chebyshev_tiled<T, false, false>);
-    return;
+    const long long waves = (columns * grid.z + wave - 1) / wave;
+    // The grid's second and third dimension hold 65535 tiles each.
+    if (cells >= kTiledStageFill * (waves * wave * kTileX * kTileY * depth) &&
+        grid.y <= 65535 && grid.z <= 65535) {
+      const dim3 block(kTileX, kTileY);
+      const auto run = [&](auto kernel) {
+        launch(kernel, grid, block, 0, s, L, x, b, direction, next, previous_factor,
+               residual_factor, depth);
+      };
+      if (first && last) run(k_chebyshev_tiled<T, true, true>);
+      else if (first) run(k_chebyshev_tiled<T, true, false>);
+      else if (last) run(k_chebyshev_tiled<T, false, true>);
+      else run(k_chebyshev_tiled<T, false, false>);
+      return;
+    }
   }
   launch(k_chebyshev_stage<T>, grid_for(cells), kThreads, 0, s, L, x, b, direction, next,
          previous_factor, residual_factor, first ? 1 : 0, last ? 1 : 0);

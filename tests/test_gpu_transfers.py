@@ -57,20 +57,27 @@ def test_prolongation_with_first_step_matches_restatement(cuda_library, shape, p
     assert np.array_equal(z, oracle.apply_mg(r))
 
 
-@pytest.mark.parametrize("shape", [(103, 101, 107), (40, 163, 165)])
+@pytest.mark.parametrize("shape,mixed_bar", [((125, 249, 121), 1e-5), ((64, 63, 468), 1e-4)])
 @pytest.mark.parametrize("pre,post", [(3, 1), (1, 3)])
-def test_tiled_stages_match_restatement(cuda_library, shape, pre, post):
-    """Chebyshev stages over 3-D tiles, levels of at least 2^20 cells: tiles cut
-    in every direction, and the first, middle and last stage and the only one."""
+def test_tiled_stages_match_restatement(cuda_library, shape, mixed_bar, pre, post):
+    """FP32 Chebyshev stages over 3-D tiles, on levels that fill three quarters of
+    a wave of them: tiles cut in every direction, and the first, middle and last
+    stage and the only one.  FP64 stages are flat and equal bit for bit.  A FP32
+    diagonal is rounded apart from its faces, which adds or takes up to u of it and
+    so moves the smoothest mode along n cells by up to u n^2 4 / pi^2 (1.5e-3 and
+    5.3e-3 here); the roundings are of either sign, and the bars are four times the
+    distance measured, 2.3e-6 and 2.5e-5."""
     import c_oracle
     import hfps
     import ref_oracle
     s = workloads.make("sphere64", n=shape, seed=6)
-    assert s.cells >= 1 << 20
     policy = hfps.Policy.production().replace(pre_sweeps=pre, post_sweeps=post,
                                               anisotropy_threshold=1e3)
     mg = ref_oracle.MgPolicy(smoother=1, cycle=1, pre=pre, post=post, diagonal_shortcut=0.1,
                              anisotropy_threshold=1e3)
     r = np.ascontiguousarray(workloads.normals(3, s.cells).reshape(s.rhs.shape))
-    z = hfps.PressureSolver.from_system(s, policy).apply_preconditioner(r)
-    assert np.array_equal(z, c_oracle.OracleSession(s, mg, unit_linear=True).apply_mg(r))
+    g = hfps.PressureSolver.from_system(s, policy)
+    expected = c_oracle.OracleSession(s, mg, unit_linear=True).apply_mg(r)
+    assert np.array_equal(g.apply_preconditioner(r), expected)
+    mixed = g.apply_preconditioner(r, precision=hfps.MIXED)
+    assert np.linalg.norm(mixed - expected) <= mixed_bar * np.linalg.norm(expected)
