@@ -915,6 +915,18 @@ void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T*
   sh.lines = threads / sh.chunks;
   while (sh.lines > threads / 32 && per_color < 592LL * sh.lines)
     sh.lines = std::max(threads / 32, sh.lines / 2);
+  // A multiple of the warps, or some load a line more than the others (FP64 pass with 9
+  // and 8 lines a block at 213x168x138 88 and 71 us, FP32 52 and 37; with 6 and 4 at
+  // 300x200x200 FP64 175 and 123): the nearest, and in FP64 two a warp rather than one
+  // (40x80x80 with 5, 4 and 8 lines 7.9, 9.3 and 7.2); less than two thirds of the lines
+  // cost more than the unevenness (138x175x163 FP32 with 14 and 8 lines 27.5 and 30.2).
+  constexpr int warps = threads / 32;
+  if (sh.lines > warps) {
+    const int up = sizeof(T) == 8 && sh.lines < 2 * warps ? warps - 1 : warps / 2;
+    const int nearest = (sh.lines + up) / warps * warps, fewer = sh.lines / warps * warps;
+    if (nearest * sh.chunks <= threads) sh.lines = nearest;
+    else if (3 * fewer >= 2 * sh.lines) sh.lines = fewer;
+  }
   constexpr size_t arrays = 1 + ScanConfig<T>::arrays;
   const size_t smem =
       static_cast<size_t>(sh.lines) * sh.chunks * (arrays * sh.pitch + 4) * sizeof(T);
