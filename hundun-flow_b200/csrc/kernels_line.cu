@@ -912,20 +912,30 @@ void launch_scan_x(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T*
   sh.chunks = (L.nx + rows - 1) / rows;
   sh.rows = (L.nx + sh.chunks - 1) / sh.chunks;
   sh.pitch = sh.rows | 1;
-  sh.lines = threads / sh.chunks;
+  // FP64 blocks of more than about 80 chunks take so much shared memory that the few
+  // of them on an SM leave loads waiting for scans (110x243x107 69 us a pass, 51 before
+  // the x scan; 47 so).  Lines of up to 3 chunks want the threads for their loads
+  // (24x300x300 34 and 42 us), those of more than 32 the lines (520x160x160 159 and 185).
+  const int most = sizeof(T) == 8 && sh.chunks > 3 && sh.chunks <= 32 ? 80 : threads;
+  sh.lines = std::max(1, most / sh.chunks);
   while (sh.lines > threads / 32 && per_color < 592LL * sh.lines)
     sh.lines = std::max(threads / 32, sh.lines / 2);
-  // A multiple of the warps, or some load a line more than the others (FP64 pass with 9
-  // and 8 lines a block at 213x168x138 88 and 71 us, FP32 52 and 37; with 6 and 4 at
-  // 300x200x200 FP64 175 and 123): the nearest, and in FP64 two a warp rather than one
-  // (40x80x80 with 5, 4 and 8 lines 7.9, 9.3 and 7.2); less than two thirds of the lines
-  // cost more than the unevenness (138x175x163 FP32 with 14 and 8 lines 27.5 and 30.2).
+  // A multiple of the warps, or some load a line more than the others (213x168x138 with
+  // 9 and 8 lines a block 88 and 71 us, FP32 52 and 37; 300x200x200 with 6 and 4 175 and
+  // 123); two a warp rather than one where they fit (40x80x80 with 5, 4 and 8 lines 7.9,
+  // 9.3 and 7.2).  FP32 blocks lose from fewer lines unless the last round was mostly
+  // empty (138x175x163 with 14 and 8 lines 26.4 and 30.2, 100x150x150 with 19 and 16
+  // 17.8 and 19.1).
   constexpr int warps = threads / 32;
-  if (sh.lines > warps) {
-    const int up = sizeof(T) == 8 && sh.lines < 2 * warps ? warps - 1 : warps / 2;
-    const int nearest = (sh.lines + up) / warps * warps, fewer = sh.lines / warps * warps;
-    if (nearest * sh.chunks <= threads) sh.lines = nearest;
-    else if (3 * fewer >= 2 * sh.lines) sh.lines = fewer;
+  if (sizeof(T) == 8 && sh.lines > warps) {
+    if (sh.lines >= 2 * warps) sh.lines = sh.lines / warps * warps;
+    else sh.lines = 2 * warps * sh.chunks <= most + 8 ? 2 * warps : warps;
+  } else if (sh.lines > warps) {
+    const int nearest = (sh.lines + warps / 2) / warps * warps;
+    const int lines = nearest * sh.chunks <= most ? nearest : sh.lines / warps * warps;
+    const int rounds = (sh.lines + warps - 1) / warps;
+    const bool uneven = 5 * rounds * warps >= 7 * sh.lines;
+    if (uneven ? 3 * lines >= 2 * sh.lines : 10 * lines >= 9 * sh.lines) sh.lines = lines;
   }
   constexpr size_t arrays = 1 + ScanConfig<T>::arrays;
   const size_t smem =
