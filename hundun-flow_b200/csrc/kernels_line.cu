@@ -856,15 +856,17 @@ ScanShape scan_shape(long long per_color, int extent) {
   return sh;
 }
 
-// Without end terms the FP64 kernel needs 128 registers instead of 165, so four
-// blocks share an SM: a level-0 pass of the split 256^3 level went from 144 to
-// 122 us and one of level 1 from 43 to 35.  In natural order the fourth block's
-// half-used sectors cost more than it gives (456x256x52 y-lines 65.6 -> 71 us),
-// and levels that three blocks per SM hold anyway gain nothing (64x256x64 9.9 ->
-// 11.0 us, 32x256x32 7.3 -> 8.3): those keep the kernel with the end terms,
-// which are exact zeros then.  FP32 has 64 registers and two blocks per SM either
-// way, and its level-0 pass is slower without them (94.5 -> 100.3 us).  A fresh pass
-// reads nothing but rhs in either form.
+// Without end terms the FP64 kernel needs 128 registers instead of 165: 16 resident
+// warps per SM, not 12.  Along y that pays where the colour's blocks then take fewer
+// waves (level-0 pass of 256^3 142 -> 123 us, 128x256x128 42 -> 36, 128^3 15.5 ->
+// 10.8, 250x140x200 78 -> 70) and costs a little where they do not (128x192x128 29.1
+// -> 30.2 us, 131x160x133 27.0 -> 27.9, 64x256x64 7.7 -> 8.0).  Along z it gained in
+// one of seventeen shapes (256^3 162 either way, 128x256x256 76 -> 81, 256x256x160 96
+// -> 100), and in natural order the half-used sectors of the fourth block cost more
+// than it gives (456x256x52 y-lines 65.6 -> 71 us).  Those keep the kernel with the
+// end terms, which are exact zeros then.  FP32 has 64 registers and two blocks per SM
+// either way, and its level-0 pass is slower without them (94.5 -> 100.3 us).  A fresh
+// pass reads nothing but rhs in either form.
 struct ScanFlags {
   int hx;
   bool zero_other, zero_self, ends;
@@ -882,8 +884,12 @@ void launch_scan(cudaStream_t s, const Level<T>& L, T* x, const T* b, const T* f
   };
   // The kernel without end terms takes the zero flag as an argument (a kernel of
   // its own takes more registers); with them it is a mode.
-  if constexpr (sizeof(T) == 8) {
-    if (!f.ends && split && blocks > 3 * 148 && !(f.zero_other && f.zero_self)) {
+  if constexpr (sizeof(T) == 8 && AXIS == 1) {
+    const int warps = (LPB * sh.chunks + 31) / 32;
+    const int resident = 148 * (12 / warps), resident_none = 148 * (16 / warps);
+    const bool fewer_waves =
+        (blocks + resident_none - 1) / resident_none < (blocks + resident - 1) / resident;
+    if (!f.ends && split && fewer_waves && !(f.zero_other && f.zero_self)) {
       run(k_line_scan_color<T, AXIS, LPB, kScanNormal, true, false>);
       return;
     }

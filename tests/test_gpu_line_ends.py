@@ -11,12 +11,13 @@ from test_gpu_parity import stretched_front
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("oracle_built")]
 
 
-# The kernel without end terms serves split rows (y- and z-lines) with more than
-# 444 blocks a colour: 131x160x133 and 131x133x160 have 8778 lines a colour, 8 a
-# block; the smaller grids keep the kernel with the end terms.
+# The kernel without end terms serves y-lines in split rows whose blocks then take
+# fewer waves: 101x150x99 has 5049 lines a colour, 8 a block of 3 warps, 632 blocks
+# where 592 are resident with end terms and 740 without; 131x256x67 has 4422, 553
+# blocks of 4 warps, 444 and 592.  The other grids keep the kernel with the end terms.
 @pytest.mark.parametrize("shape,axis", [
     ((60, 48, 48), 0), ((48, 60, 48), 1), ((48, 48, 60), 2),
-    ((131, 160, 133), 1), ((131, 133, 160), 2)])
+    ((101, 150, 99), 1), ((131, 256, 67), 1), ((131, 133, 160), 2)])
 @pytest.mark.parametrize("face", [0.0, 0.3])
 def test_neumann_faces_at_line_ends(cuda_library, shape, axis, face):
     import c_oracle
