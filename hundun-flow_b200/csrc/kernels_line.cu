@@ -392,10 +392,10 @@ __global__ void __launch_bounds__(ScanConfig<T>::threads)
 // the factors follow by asynchronous copies that hold no registers, each
 // thread then scans its chunk of up to ScanConfig<T>::rows rows out of shared
 // memory (chunks padded to an odd length, so that the lanes of a line fall in
-// different banks), and the solution goes back coalesced: 76 us, 2.8 TB/s of
+// different banks), and the solution goes back coalesced: 75 us, 2.9 TB/s of
 // the 36 bytes per cell that a pass needs (the transverse faces are 16 of them,
-// the factors 8).  A block of at most 2048 rows takes 52 KB of shared memory,
-// so that four blocks per SM overlap their load and scan phases; what bounds
+// the factors 8).  A FP64 block of some 1280 rows takes 35 KB of shared memory,
+// so that six blocks per SM overlap their load and scan phases; what bounds
 // it now is the rest of that overlap.  Chunks, compositions and their
 // order are k_line_scan_color's, so the results are bit for bit its results.
 constexpr int kScanXThreads = 128;
